@@ -22,7 +22,6 @@ constexpr int NPE_MAX = 256;   // extended cell parts (q0+1)(q1+1)(q2+1)
 constexpr int OCCW_MAX = 4;    // 64-bit part-occupancy words per cell
 constexpr int ARRCAP = 32;     // arrival slots per cell before the overflow list
 constexpr int CELL_WARPS = 4;  // warps per block of the warp-per-cell helper kernels
-constexpr int KEY_CACHE = 128; // (part, key) pairs cached per warp on the general path
 constexpr int ADV_CH = 512;    // particles per staged chunk of the FP32 advect pass
 // cells whose velocity records an FP32 advect chunk stages with its particles
 // (a chunk spans about ADV_CH / particles-per-cell + 1 cells; beyond this
@@ -30,8 +29,6 @@ constexpr int ADV_CH = 512;    // particles per staged chunk of the FP32 advect 
 template <int DIM> struct AdvRec {
     static constexpr int MAXC = DIM == 3 ? 32 : 48;
 };
-constexpr int WR_WARPS = 4;    // write pass: warps per block
-constexpr int WR_CHC = 4;      // write pass: cells per warp chunk
 
 // error_flags bits
 constexpr uint32_t ERR_CAPACITY = 1u;        // more particles than the arrays hold
@@ -57,8 +54,8 @@ struct DevStats {
     unsigned long long step_holes;   // empty slots left by the last write pass
     unsigned int next_id;
     unsigned int error_flags;
-    unsigned int write_done;         // write pass: warps finished (the last one finalises the step)
-    unsigned int write_next;         // write pass: next chunk of cells to hand out
+    unsigned int write_done;         // write pass: blocks finished (the last one finalises the step)
+    unsigned int write_next;         // write pass: next tile of cells to hand out
     unsigned int adv_next;           // advect pass: next chunk of particles to hand out
 };
 

@@ -6,6 +6,7 @@
 #include "cellwork.cuh"
 #include "launch.h"
 #include "shard.cuh"
+#include "write.cuh"
 
 namespace pfem2 {
 
@@ -145,27 +146,12 @@ int launch64_cross(int dim, const StepArgs& a, cudaStream_t s)
     return dim == 2 ? search_t<2, false>(a, s) : search_t<3, false>(a, s);
 }
 
-template <int DIM, int CHC>
-static int write_c(const StepArgs& a, cudaStream_t s)
-{
-    const int smem = WR_WARPS * (int)sizeof(WrWarp<DIM, double>);
-    // bulk-copy staging where a chunk of cells at the seeding density fits the stage
-    if (CHC * a.pp.npart <= WrCfg<DIM, double>::UCAP) {
-        static const int grid = smem_grid(k_write<DIM, double, true, CHC>, WR_WARPS * 32, smem);
-        return launch_pdl(k_write<DIM, double, true, CHC>, grid, WR_WARPS * 32, smem, s, a);
-    }
-    static const int grid = smem_grid(k_write<DIM, double, false, CHC>, WR_WARPS * 32, smem);
-    return launch_pdl(k_write<DIM, double, false, CHC>, grid, WR_WARPS * 32, smem, s, a);
-}
-
-// Chunks of 4 cells on affine meshes; of 2 on the others (graded and
-// unstructured meshes, whose cells differ most in particles and arrivals:
-// smaller chunks spread the busiest cells over more warps).
 template <int DIM>
 static int write_t(const StepArgs& a, cudaStream_t s)
 {
-    if (a.mesh.all_affine) return write_c<DIM, WrCfg<DIM, double>::CHC>(a, s);
-    return write_c<DIM, WrCfg<DIM, double>::CHC_UNEVEN>(a, s);
+    const int smem = (int)sizeof(WtTile<DIM, double>);
+    static const int grid = smem_grid(k_write<DIM, double>, WT_THREADS, smem);
+    return launch_pdl(k_write<DIM, double>, grid, WT_THREADS, smem, s, a);
 }
 
 int launch64_write(int dim, const StepArgs& a, cudaStream_t s)

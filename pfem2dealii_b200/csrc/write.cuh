@@ -1,0 +1,744 @@
+// The write pass: count correction, the new sorted layout, projection partial
+// sums and the step's counters, in one kernel.
+//
+// A block takes a tile of consecutive cells, whose old slots are one range of
+// the arrays.  The range is bulk-copied into shared memory, the cells'
+// arrivals are gathered behind it, and the block then works on these entries
+// one per thread: part counts, survivors of over-full parts (by key), places
+// in the new layout (stayers by a prefix of their survival bits, arrivals by
+// their key), stores.  Nothing is read from global memory twice, and a
+// warp's lanes are all in use whatever a cell holds.  At last a warp per cell
+// takes the partial sums from the staged entries in the new order.
+//
+// What bounds it, and why tiles.  A time step's memory traffic here is 69
+// bytes a particle (FP32, 3D).  One warp per cell with one register round per
+// 32 particles (the layout before) lost its lanes to cells of 33 or 97
+// particles, could stage four cells only at seeding density, re-read the
+// written particles for the partial sums of cells above 32, and sent cells
+// above 96 to a path that counts positions through global scratch.  A run
+// settles near 1.9 particles per part (54 a cell at 27 parts, 124 at 64), so
+// those were the paths in use.
+#pragma once
+
+#include "cellwork.cuh"
+
+namespace pfem2 {
+
+template <int DIM, typename Real>
+struct PData {
+    uint32_t i, id;
+    Real xi[DIM], v[DIM];
+    Real x[std::is_same<Real, double>::value ? DIM : 1];
+};
+
+template <int DIM, typename Real>
+__device__ __forceinline__ void load_global(const StepArgs& a, uint32_t i, PData<DIM, Real>& p)
+{
+    p.i = i;
+    p.id = a.S0.id[i];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        p.xi[d] = ldr<Real>(a.T.xi[d], i);
+        p.v[d] = ldr<Real>(a.T.v[d], i);
+        if constexpr (std::is_same<Real, double>::value) p.x[d] = ldr<double>(a.T.x[d], i);
+    }
+}
+
+template <int DIM, typename Real>
+__device__ __forceinline__ void store_particle(const StepArgs& a, uint32_t dst, uint32_t c, const PData<DIM, Real>& p)
+{
+    a.S1.cell[dst] = c;
+    a.S1.id[dst] = p.id;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        str<Real>(a.S1.xi[d], dst, p.xi[d]);
+        str<Real>(a.S1.v[d], dst, p.v[d]);
+        if constexpr (std::is_same<Real, double>::value) str<double>(a.S1.x[d], dst, p.x[d]);
+    }
+}
+
+// Empty slots [from, to) of a cell's range.
+__device__ __forceinline__ void write_holes(const StepArgs& a, uint32_t from, uint32_t to, int lane)
+{
+    for (uint32_t j = from + lane; j < to; j += 32)
+        if (j < a.capacity) a.S1.cell[j] = HOLE;
+}
+
+// New particles of one cell (one warp): the k-th seeded part (in part order)
+// goes to slot base + k and gets id id0 + sb + k + 1; stage(k, xi, v) sees it.
+// Returns the number of new particles and error bits.
+template <int DIM, typename Real, typename F>
+__device__ __forceinline__ uint2 write_seeds(const StepArgs& a, uint32_t c, const int* cnt, uint32_t n, uint32_t base,
+                                             uint32_t id0, uint32_t sb, int lane, F&& stage)
+{
+    uint32_t done = 0, err = 0;
+    for (int p0 = 0; p0 < a.pp.npe; p0 += 32) {
+        const int p = p0 + lane;
+        const bool sf = p < a.pp.npe && gets_seed(a, p, cnt[p < a.pp.npe ? p : 0], n);
+        const unsigned m = __ballot_sync(0xffffffffu, sf);
+        if (sf) {
+            const uint32_t k = done + __popc(m & ((1u << lane) - 1u));
+            const uint32_t dst = base + k;
+            int idx[3] = {0, 0, 0};
+            real_part<DIM>(p, a.pp, idx);
+            Real xi[DIM], v[DIM];
+            if (dst < a.capacity) {
+                new_particle<DIM, Real>(a, a.S1, dst, c, idx, id0 + sb + k + 1, xi, v);
+                stage(k, xi, v);
+            } else {
+                err |= ERR_CAPACITY;
+            }
+        }
+        done += __popc(m);
+    }
+    return make_uint2(done, err);
+}
+
+// One cell of any particle count (one warp), for the cells that fit no tile.
+// Per-element data goes to the cell's own slot range of the scratch array;
+// survivors and positions are found by counting.  Order: stayers by slot,
+// arrivals by key, new particles by part -- the same as the tiles'.
+template <int DIM, typename Real>
+__device__ __noinline__ uint2 write_cell_general(const StepArgs& a, int* cnt, Real (*tr)[TRW], uint32_t c, uint32_t s0,
+                                                 uint32_t L, uint32_t na, uint32_t h, uint32_t off, uint32_t ub,
+                                                 uint32_t nseed_expect, uint32_t sb, uint32_t id0, int lane)
+{
+    uint32_t removed = 0, err = 0;
+    uint4* G = a.gscr + off;  // element -> (particle index, part, key, flags: 1 stayer, 2 survivor)
+    const int npe = a.pp.npe;
+    for (int p = lane; p < npe; p += 32) cnt[p] = 0;
+    __syncwarp();
+    if (off + ub > a.capacity) return make_uint2(0u, ERR_CAPACITY);
+    // stayers: elements 0..ns-1 in slot order
+    uint32_t ns = 0;
+    for (uint32_t base = 0; base < L; base += 32) {
+        const uint32_t j = base + lane;
+        const bool stay = j < L && a.key[s0 + j] == c;
+        const unsigned m = __ballot_sync(0xffffffffu, stay);
+        if (stay) {
+            const uint32_t i = s0 + j, e = ns + __popc(m & ((1u << lane) - 1u));
+            Real xi[DIM];
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) xi[d] = ldr<Real>(a.T.xi[d], i);
+            const int pe = ext_part<DIM, Real>(xi, a.pp);
+            if (e < ub) G[e] = make_uint4(i, (uint32_t)pe, key_of(a.S0.id[i], a.pp.seed), 1u);
+            atomicAdd(cnt + pe, 1);
+        }
+        ns += __popc(m);
+    }
+    // arrivals: elements ns.. (slots lane-parallel; the overflow list walked by all lanes)
+    uint32_t t = 0, p = h;
+    for (; t < na && t < a.capacity; ++t) {
+        uint32_t i;
+        if (t < (uint32_t)ARRCAP) {
+            i = a.carrs[(size_t)c * ARRCAP + t];
+        } else {
+            if (p == LOST) break;
+            i = p;
+            p = a.next[p];
+        }
+        if ((t & 31u) == (uint32_t)lane) {
+            Real xi[DIM];
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) xi[d] = ldr<Real>(a.T.xi[d], i);
+            const int pe = ext_part<DIM, Real>(xi, a.pp);
+            if (ns + t < ub) G[ns + t] = make_uint4(i, (uint32_t)pe, key_of(a.S0.id[i], a.pp.seed), 0u);
+            atomicAdd(cnt + pe, 1);
+        }
+    }
+    const uint32_t n = ns + t;
+    __syncwarp();
+    __threadfence_block();
+    if (n > ub) return make_uint2(0u, ERR_COUNT_UB);
+    // survivors: rank by key inside the part
+    uint32_t nsurv = 0;
+    for (uint32_t e = lane; e < n; e += 32) {
+        const uint4 g = G[e];
+        const int k = cnt[g.y];
+        int rank = 0;
+        if (a.apply_counts && k > a.pp.maxpp + 1)
+            for (uint32_t m = 0; m < n; ++m) {
+                const uint4 o = G[m];
+                rank += (o.y == g.y && o.z < g.z) ? 1 : 0;
+            }
+        if (rank < survivors(k, a.pp.maxpp, a.apply_counts)) {
+            G[e].w = g.w | 2u;
+            nsurv++;
+        } else {
+            removed++;
+        }
+    }
+    nsurv = __reduce_add_sync(0xffffffffu, nsurv);
+    __syncwarp();
+    __threadfence_block();
+    // positions: survivors before in (stayers by slot | arrivals by key) order
+    for (uint32_t e = lane; e < n; e += 32) {
+        const uint4 g = G[e];
+        if (!(g.w & 2u)) continue;
+        const bool gs = g.w & 1u;
+        uint32_t pos = 0;
+        for (uint32_t m = 0; m < n; ++m) {
+            const uint4 o = G[m];
+            if (!(o.w & 2u)) continue;
+            const bool os = o.w & 1u;
+            pos += ((os && !gs) || (os && gs && o.x < g.x) || (!os && !gs && o.z < g.z)) ? 1u : 0u;
+        }
+        PData<DIM, Real> pd;
+        load_global<DIM, Real>(a, g.x, pd);
+        store_particle<DIM, Real>(a, off + pos, c, pd);
+    }
+    const uint2 sd = write_seeds<DIM, Real>(a, c, cnt, n, off + nsurv, id0, sb, lane,
+                                            [](uint32_t, const Real*, const Real*) {});
+    err |= sd.y;
+    const uint32_t nseed = sd.x;
+    const uint32_t fin = nsurv + nseed;
+    if (nseed != nseed_expect) err |= ERR_COUNT;
+    if (fin > ub) err |= ERR_COUNT_UB;
+    write_holes(a, off + fin, off + ub, lane);
+    __syncwarp();
+    __threadfence_block();
+    partials_of_range<DIM, Real>(a, a.S1, c, off, fin < ub ? fin : ub, tr, lane);
+    return make_uint2(removed, err);
+}
+
+// A cell's new range [off, off + ub), within the capacity, and the advect
+// chunks that start in it.
+__device__ __forceinline__ void new_range(const StepArgs& a, uint32_t c, uint32_t off, uint32_t ub)
+{
+    const uint32_t first = off < a.capacity ? off : a.capacity, end = ub < a.capacity - first ? first + ub : a.capacity;
+    a.cs_new[c] = first;
+    if (a.chunk_first)
+        for (uint32_t k = (first + ADV_CH - 1) / ADV_CH; (uint64_t)k * ADV_CH < end; ++k) a.chunk_first[k] = c;
+}
+
+// FP32 partial sums of up to 32 particles, one per lane (lanes without a
+// particle add zeros): a pairwise tree over the 32 rows, then one compensated
+// add into acc (lane = entry).  The first level of the tree, rows
+// u + (u + 16), is taken through one shuffle instead of shared memory: lane
+// u < 16 keeps the entries of the vertices whose highest reference-coordinate
+// bit is clear, lane u + 16 those with it set, and receives them from its
+// partner, so each entry crosses the warp once and 16 rows of PW entries are
+// staged; the tree's other levels follow.  Shape values and products are
+// those of partial_row (N = (x0 factor * x1 factor) * x2 factor).  EXACT:
+// every product is rounded before it is added, as partial_row's are.
+template <int DIM, bool EXACT>
+__device__ __forceinline__ void partial_pairs32(float (*tr)[TRW], bool active, const float* xi, const float* v,
+                                                int lane, PartialAcc<float>& acc)
+{
+    constexpr int NV = 1 << DIM, H = NV / 2, PW = Dims<DIM>::PW;
+    const bool hi = lane >= 16;
+    float x[DIM], w[DIM];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        x[d] = active ? xi[d] : 0.0f;
+        w[d] = active ? v[d] : 0.0f;
+    }
+    float lowN[H];  // products of the factors below the highest direction
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+        float n = (k & 1) ? x[0] : 1.0f - x[0];
+        if (DIM > 2) n *= ((k >> 1) & 1) ? x[1] : 1.0f - x[1];
+        lowN[k] = n;
+    }
+    // a lane without a particle adds nothing (its shape values are zero too)
+    const float top = x[DIM - 1], bot = 1.0f - x[DIM - 1];
+    const float fk = active ? (hi ? top : bot) : 0.0f, fs = active ? (hi ? bot : top) : 0.0f;
+    float keep[4 * H];
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+        const float nk = EXACT ? __fmul_rn(lowN[k], fk) : lowN[k] * fk;
+        const float ns = EXACT ? __fmul_rn(lowN[k], fs) : lowN[k] * fs;
+        float e[4], f[4];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            e[d] = EXACT ? __fmul_rn(nk, w[d]) : nk * w[d];
+            f[d] = EXACT ? __fmul_rn(ns, w[d]) : ns * w[d];
+        }
+        e[DIM] = nk;
+        f[DIM] = ns;
+        if (DIM == 2) e[3] = f[3] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) keep[4 * k + j] = e[j] + __shfl_xor_sync(0xffffffffu, f[j], 16);
+    }
+    const int row = lane & 15, col0 = hi ? 4 * H : 0;
+#pragma unroll
+    for (int k = 0; k < H; ++k)
+        *reinterpret_cast<float4*>(&tr[row][col0 + 4 * k]) =
+            make_float4(keep[4 * k], keep[4 * k + 1], keep[4 * k + 2], keep[4 * k + 3]);
+    __syncwarp();
+    if (lane < PW) {
+        float t[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) t[r] = tr[r][lane];
+#pragma unroll
+        for (int wd = 8; wd >= 1; wd >>= 1)
+#pragma unroll
+            for (int r = 0; r < wd; ++r) t[r] = t[r] + t[r + wd];
+        const float y = t[0] - acc.c;
+        const float sm = acc.s + y;
+        acc.c = (sm - acc.s) - y;
+        acc.s = sm;
+    }
+}
+
+// FP64 partial sums of one cell, in particle order (as the oracle adds them),
+// without shared rows: lane = entry (vertex lane / 4, component lane % 4).
+// Four particles at a time: the four lanes of a vertex take its shape value
+// of one particle each and exchange them by shuffles, and every lane adds its
+// component of the four in order.  2D has 16 entries; the upper lanes repeat
+// the lower ones' work.  at(r) = the staged entry of the r-th particle.
+template <int DIM, int CAP, typename At>
+__device__ __forceinline__ double partial_seq64(const double (*xi)[CAP], const double (*v)[CAP], uint32_t fin, int lane,
+                                                At&& at)
+{
+    const int iv = (lane >> 2) & ((1 << DIM) - 1), comp = lane & 3;
+    double acc = 0.0;
+    for (uint32_t r0 = 0; r0 < fin; r0 += 4) {
+        const uint32_t own = at(r0 + comp < fin ? r0 + comp : r0);
+        double N = lag64(iv & 1, xi[0][own]);
+        N = N * lag64((iv >> 1) & 1, xi[1][own]);
+        if (DIM > 2) N = N * lag64((iv >> 2) & 1, xi[DIM - 1][own]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const double Nj = __shfl_sync(0xffffffffu, N, (lane & ~3) | j);
+            const uint32_t e = __shfl_sync(0xffffffffu, own, (lane & ~3) | j);
+            if (r0 + j < fin) {
+                const double t = comp < DIM ? Nj * v[comp < DIM ? comp : 0][e] : (comp == DIM ? Nj : 0.0);
+                acc = acc + t;
+            }
+        }
+    }
+    return acc;
+}
+
+// ---------------------------------------------------------------------------
+// Tiles.  TCAP entries (old slots, arrivals, new particles) fit one tile's
+// shared memory: 6 blocks of 128 threads per SM in the FP32 form, 4 in the
+// FP64 form.  The kernel takes as many cells per tile as bring it near TARGET
+// particles at the layout's mean density, fewer where the tiles would not
+// fill the grid; a tile that holds more than TCAP is worked through in runs
+// of cells that fit, and a single cell beyond TCAP takes the general path.
+// ---------------------------------------------------------------------------
+constexpr int WT_WARPS = 4, WT_THREADS = WT_WARPS * 32;
+constexpr int WT_CELLS = 24;  // cells per tile at most
+constexpr int WT_CNT = 1024;  // part counters of a run of cells
+
+template <int DIM, typename Real>
+struct WtCfg {
+    static constexpr bool HX = std::is_same<Real, double>::value;
+    static constexpr int TCAP = HX ? 480 : 512;
+    static constexpr int TARGET = HX ? 440 : 470;
+};
+
+template <int DIM, typename Real>
+struct __align__(128) WtTile {
+    static constexpr bool HX = WtCfg<DIM, Real>::HX;
+    static constexpr int TCAP = WtCfg<DIM, Real>::TCAP;
+    uint32_t key[TCAP];  // the move's cell, then key_of(id)
+    uint32_t id[TCAP];
+    Real xi[DIM][TCAP];
+    Real v[DIM][TCAP];
+    Real x[HX ? DIM : 1][HX ? TCAP : 4];
+    Real tr[HX ? 1 : WT_WARPS][HX ? 1 : 16][TRW];  // FP32 partial rows, one block of 16 per warp
+    int cnt[WT_CNT];
+    uint16_t meta[TCAP];  // local cell << 8 | extended part; 0xffff: not in the new layout
+    uint16_t perm[TCAP];  // over-full parts' entries, then the entry of each new slot
+    uint32_t mask[TCAP / 32 + 1];  // survivors
+    uint32_t cs[WT_CELLS + 1], aoff[WT_CELLS + 1], off[WT_CELLS + 1], sb[WT_CELLS + 1];
+    uint32_t head[WT_CELLS], occ[WT_CELLS];
+    uint64_t bar;
+    uint32_t ticket, nover;
+};
+
+template <int DIM, typename Real>
+__global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ StepArgs a)
+{
+    constexpr bool HX = WtCfg<DIM, Real>::HX;
+    constexpr int TCAP = WtCfg<DIM, Real>::TCAP, TARGET = WtCfg<DIM, Real>::TARGET;
+    static_assert(TCAP % 32 == 0 && TCAP / 32 < 32, "one survivor word per lane");
+    extern __shared__ __align__(128) unsigned char wr_raw[];
+    auto& w = *reinterpret_cast<WtTile<DIM, Real>*>(wr_raw);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        mbar_init(&w.bar, 1);
+        mbar_fence_init();
+        w.nover = 0;
+    }
+    pdl_entry();
+    const uint32_t nC = (uint32_t)a.mesh.nC, cap = a.capacity;
+    const uint32_t id0 = a.stats->next_id;
+    const int apply = a.apply_counts, maxpp = a.pp.maxpp, npe = a.pp.npe;
+    uint32_t NC;  // cells per tile
+    {
+        const unsigned long long total = a.coff[nC] & 0xffffffffull;
+        const unsigned long long by_load = total ? (unsigned long long)TARGET * nC / total : WT_CELLS;
+        const uint32_t by_grid = (nC + gridDim.x - 1) / gridDim.x, by_cnt = WT_CNT / npe;
+        NC = by_load < WT_CELLS ? (uint32_t)by_load : WT_CELLS;
+        NC = min(min(NC, by_grid), by_cnt);
+        NC = NC < 1 ? 1 : NC;
+    }
+    const uint32_t ntiles = (nC + NC - 1) / NC;
+    unsigned long long removed = 0;
+    uint32_t err = 0, phase = 0;
+    bool stage_ok = true;  // cleared for good if a copy ever fails to land in time
+    if (tid == 0) w.ticket = atomicAdd(&a.stats->write_next, 1u);
+    while (true) {
+        __syncthreads();
+        const uint32_t tile = w.ticket;
+        if (tile >= ntiles) break;
+        const uint32_t c0 = tile * NC, ncell = nC - c0 < NC ? nC - c0 : NC;
+        uint32_t next_ticket = 0;
+        if (warp == 0) {  // the cells' headers, one cell per lane; their counters are reset for the next move
+            const bool in = (uint32_t)lane < ncell;
+            const uint32_t c = c0 + lane;
+            uint32_t na = 0;
+            if ((uint32_t)lane <= ncell) {
+                const unsigned long long o = a.coff[c];
+                w.cs[lane] = a.cs_old[c];
+                w.off[lane] = (uint32_t)o;
+                w.sb[lane] = (uint32_t)(o >> 32);
+            }
+            if (in) {
+                na = a.carr[c];
+                w.head[lane] = a.head[c];
+                uint32_t occ = 0;
+                for (int q = 0; q < a.pp.occw; ++q) {
+                    occ += __popcll(a.cocc[(size_t)c * a.pp.occw + q]);
+                    a.cocc[(size_t)c * a.pp.occw + q] = 0ull;
+                }
+                w.occ[lane] = occ;
+                a.carr[c] = 0;
+                a.ccount[c] = 0;
+                a.head[c] = LOST;
+            }
+            uint32_t inc = na;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            if ((uint32_t)lane <= ncell) w.aoff[lane] = inc - na;
+            if (lane == 0) next_ticket = atomicAdd(&a.stats->write_next, 1u);
+        }
+        __syncthreads();
+        if (tid == 0) w.ticket = next_ticket;
+        for (uint32_t cb = 0; cb < ncell;) {
+            // the longest run of cells [cb, ce) that fits
+            const uint32_t SA = w.cs[cb] & ~3u;
+            uint32_t ce;
+            {
+                const uint32_t j = cb + 1 + lane;
+                bool fits = false;
+                if (j <= ncell) {
+                    const uint32_t ent = ((w.cs[j] + 3u) & ~3u) - SA + (w.aoff[j] - w.aoff[cb]) + (w.sb[j] - w.sb[cb]);
+                    fits = ent <= (uint32_t)TCAP && w.off[j] - w.off[cb] <= (uint32_t)TCAP;
+                }
+                ce = cb + (uint32_t)__popc(__ballot_sync(0xffffffffu, fits));
+            }
+            if (ce == cb) {  // a single cell beyond a tile
+                if (warp == 0) {
+                    const uint32_t c = c0 + cb, off = w.off[cb], ub = w.off[cb + 1] - off;
+                    // its rows live where a tile's entries would
+                    auto* tr = reinterpret_cast<Real(*)[TRW]>(HX ? (void*)&w.xi[0][0] : (void*)&w.tr[0][0][0]);
+                    const uint2 gr = write_cell_general<DIM, Real>(a, w.cnt, tr, c, w.cs[cb], w.cs[cb + 1] - w.cs[cb],
+                                                                   w.aoff[cb + 1] - w.aoff[cb], w.head[cb], off, ub,
+                                                                   w.sb[cb + 1] - w.sb[cb], w.sb[cb], id0, lane);
+                    if (lane == 0) new_range(a, c, off, ub);
+                    removed += gr.x;
+                    err |= gr.y;
+                }
+                ce = cb + 1;
+            } else {
+                const uint32_t E = w.cs[ce], EA = (E + 3u) & ~3u;
+                const uint32_t nold = w.cs[cb] < E ? EA - SA : 0u, a0 = w.aoff[cb], narr = w.aoff[ce] - a0;
+                const uint32_t nE = nold + narr, nch = (nE + 31u) >> 5;
+                if (nold) {
+                    if (stage_ok) {
+                        if (tid == 0) {
+                            fence_proxy_async();  // the previous run's reads come first
+                            constexpr uint32_t per = 8u + 2u * DIM * sizeof(Real) + (HX ? DIM * 8u : 0u);
+                            mbar_expect_tx(&w.bar, nold * per);
+                            bulk_g2s(w.key, a.key + SA, nold * 4u, &w.bar);
+                            bulk_g2s(w.id, a.S0.id + SA, nold * 4u, &w.bar);
+#pragma unroll
+                            for (int d = 0; d < DIM; ++d) {
+                                bulk_g2s(w.xi[d], reinterpret_cast<const Real*>(a.T.xi[d]) + SA,
+                                         nold * (uint32_t)sizeof(Real), &w.bar);
+                                bulk_g2s(w.v[d], reinterpret_cast<const Real*>(a.T.v[d]) + SA,
+                                         nold * (uint32_t)sizeof(Real), &w.bar);
+                                if constexpr (HX)
+                                    bulk_g2s(w.x[d], reinterpret_cast<const double*>(a.T.x[d]) + SA, nold * 8u, &w.bar);
+                            }
+                        }
+                    } else {
+                        for (uint32_t j = tid; j < nold; j += WT_THREADS) {
+                            PData<DIM, Real> p;
+                            load_global<DIM, Real>(a, SA + j, p);
+                            w.key[j] = a.key[SA + j];
+                            w.id[j] = p.id;
+#pragma unroll
+                            for (int d = 0; d < DIM; ++d) {
+                                w.xi[d][j] = p.xi[d];
+                                w.v[d][j] = p.v[d];
+                                if constexpr (HX) w.x[d][j] = p.x[d];
+                            }
+                        }
+                    }
+                }
+                for (uint32_t t = tid; t < (ce - cb) * npe; t += WT_THREADS) w.cnt[t] = 0;
+                // arrivals beyond their cell's slots: one thread walks each overflow list
+                bool ovf = false;
+                if (cb + lane < ce) ovf = w.aoff[cb + lane + 1] - w.aoff[cb + lane] > (uint32_t)ARRCAP;
+                if (__any_sync(0xffffffffu, ovf)) {
+                    if (warp == 0 && ovf) {
+                        const uint32_t lc = cb + lane, na = w.aoff[lc + 1] - w.aoff[lc];
+                        uint32_t p = w.head[lc];
+                        for (uint32_t k = ARRCAP; k < na; ++k) {
+                            w.key[nold + (w.aoff[lc] - a0) + k] = p;
+                            if (p < cap) p = a.next[p];
+                        }
+                    }
+                    __syncthreads();
+                }
+                for (uint32_t t = tid; t < narr; t += WT_THREADS) {
+                    uint32_t lc = cb;
+                    while (w.aoff[lc + 1] - a0 <= t) ++lc;
+                    const uint32_t k = t - (w.aoff[lc] - a0), e = nold + t;
+                    const uint32_t i = k < (uint32_t)ARRCAP ? a.carrs[(size_t)(c0 + lc) * ARRCAP + k] : w.key[e];
+                    if (i < cap) {
+                        PData<DIM, Real> p;
+                        load_global<DIM, Real>(a, i, p);
+                        w.id[e] = p.id;
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) {
+                            w.xi[d][e] = p.xi[d];
+                            w.v[d][e] = p.v[d];
+                            if constexpr (HX) w.x[d][e] = p.x[d];
+                        }
+                        w.meta[e] = (uint16_t)(lc << 8);
+                    } else {
+                        err |= ERR_ARRIVAL;
+                        w.meta[e] = 0xffffu;
+                    }
+                }
+                if (nold && stage_ok) {
+                    if (__syncthreads_or(!mbar_wait(&w.bar, phase))) {
+                        // give the copy one more bounded wait, then stop staging; this run's particles are lost
+                        err |= ERR_TIMEOUT;
+                        mbar_wait(&w.bar, phase);
+                        stage_ok = false;
+                        __syncthreads();
+                    }
+                    phase ^= 1u;
+                } else {
+                    __syncthreads();
+                }
+                // cell, part and key of every entry; part counts
+                for (uint32_t e = tid; e < nE; e += WT_THREADS) {
+                    uint32_t m = 0xffffu;
+                    if (e < nold) {
+                        const uint32_t lc = w.key[e] - c0, slot = SA + e;
+                        if (lc >= cb && lc < ce && slot >= w.cs[lc] && slot < w.cs[lc + 1]) m = lc << 8;
+                    } else {
+                        m = w.meta[e];
+                    }
+                    if (m != 0xffffu) {
+                        Real xi[DIM];
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) xi[d] = w.xi[d][e];
+                        const int pe = ext_part<DIM, Real>(xi, a.pp);
+                        if (apply) atomicAdd(w.cnt + ((m >> 8) - cb) * npe + pe, 1);
+                        m |= (uint32_t)pe;
+                        w.key[e] = key_of(w.id[e], a.pp.seed);
+                    }
+                    w.meta[e] = (uint16_t)m;
+                }
+                __syncthreads();
+                // survivors: everyone outside the over-full parts, and there the smallest keys
+                bool over = false;
+                for (uint32_t e = tid; e < nch * 32u; e += WT_THREADS) {
+                    const uint32_t m = e < nE ? w.meta[e] : 0xffffu;
+                    bool live = m != 0xffffu;
+                    if (live && apply && w.cnt[((m >> 8) - cb) * npe + (m & 255u)] > maxpp + 1) {
+                        w.perm[atomicAdd(&w.nover, 1u)] = (uint16_t)e;
+                        over = true;
+                        live = false;
+                    }
+                    const unsigned b = __ballot_sync(0xffffffffu, live);
+                    if (lane == 0) w.mask[e >> 5] = b;
+                }
+                if (__syncthreads_or(over)) {
+                    const uint32_t nov = w.nover;
+                    for (uint32_t j = tid; j < nov; j += WT_THREADS) {
+                        const uint32_t e = w.perm[j], m = w.meta[e], kk = w.key[e];
+                        int rank = 0;
+                        for (uint32_t o = 0; o < nov; ++o) {
+                            const uint32_t f = w.perm[o];
+                            rank += (w.meta[f] == m && w.key[f] < kk) ? 1 : 0;
+                        }
+                        if (rank < maxpp + 1) atomicOr(w.mask + (e >> 5), 1u << (e & 31u));
+                        else removed++;
+                    }
+                    __syncthreads();
+                    if (tid == 0) w.nover = 0;
+                }
+                // survivors before an entry: words by a scan over the lanes, bits by a count
+                const uint32_t word = (uint32_t)lane < nch ? w.mask[lane] : 0u;
+                uint32_t wpre = __popc(word);
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, wpre, o);
+                    if (lane >= o) wpre += y;
+                }
+                wpre -= __popc(word);
+                auto before = [&](uint32_t e) {  // called by whole warps
+                    const uint32_t p = __shfl_sync(0xffffffffu, wpre, (int)(e >> 5));
+                    const uint32_t b = __shfl_sync(0xffffffffu, word, (int)(e >> 5));
+                    return p + (uint32_t)__popc(b & ((1u << (e & 31u)) - 1u));
+                };
+                // places and stores
+                const uint32_t ob = w.off[cb];
+                for (uint32_t e = tid; e < nch * 32u; e += WT_THREADS) {
+                    const uint32_t m = e < nE ? w.meta[e] : 0xffffu;
+                    const bool live = (w.mask[e >> 5] >> lane) & 1u;
+                    const uint32_t lc = live ? m >> 8 : cb;
+                    const uint32_t lb = nold ? w.cs[lc] - SA : 0u, le = nold ? w.cs[lc + 1] - SA : 0u;
+                    const uint32_t pb = before(lb), pe = before(le), ps = before(e);
+                    if (!live) continue;
+                    uint32_t pos;
+                    if (e < nold) {
+                        pos = ps - pb;
+                    } else {
+                        pos = pe - pb;
+                        const uint32_t kk = w.key[e];
+                        const uint32_t o1 = nold + w.aoff[lc + 1] - a0;
+                        for (uint32_t o = nold + w.aoff[lc] - a0; o < o1; ++o)
+                            pos += (((w.mask[o >> 5] >> (o & 31u)) & 1u) && w.key[o] < kk) ? 1u : 0u;
+                    }
+                    const uint32_t dst = w.off[lc] + pos;
+                    if (pos >= w.off[lc + 1] - w.off[lc]) {
+                        err |= ERR_COUNT_UB;
+                        continue;
+                    }
+                    w.perm[dst - ob] = (uint16_t)e;
+                    if (dst >= cap) {
+                        err |= ERR_CAPACITY;
+                        continue;
+                    }
+                    a.S1.cell[dst] = c0 + lc;
+                    a.S1.id[dst] = w.id[e];
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) {
+                        str<Real>(a.S1.xi[d], dst, w.xi[d][e]);
+                        str<Real>(a.S1.v[d], dst, w.v[d][e]);
+                        if constexpr (HX) str<double>(a.S1.x[d], dst, w.x[d][e]);
+                    }
+                }
+                // the cells' survivors, new particles and empty slots: a warp per cell, the same warp
+                // as for the sums below
+                auto survivors_of = [&](uint32_t lc, uint32_t& ns) {
+                    const uint32_t lb = nold ? w.cs[lc] - SA : 0u, le = nold ? w.cs[lc + 1] - SA : 0u;
+                    ns = before(le) - before(lb);
+                    return ns + before(nold + w.aoff[lc + 1] - a0) - before(nold + w.aoff[lc] - a0);
+                };
+                for (uint32_t lc = cb + warp; lc < ce; lc += WT_WARPS) {
+                    const uint32_t c = c0 + lc, off = w.off[lc], ub = w.off[lc + 1] - off;
+                    const uint32_t nseed = w.sb[lc + 1] - w.sb[lc];
+                    uint32_t ns;
+                    const uint32_t nsurv = survivors_of(lc, ns);
+                    if (nseed) {
+                        const uint32_t e0 = nE + (w.sb[lc] - w.sb[cb]);
+                        const uint2 sd = write_seeds<DIM, Real>(
+                            a, c, w.cnt + (lc - cb) * npe, 1u, off + nsurv, id0, w.sb[lc], lane,
+                            [&](uint32_t k, const Real* xi, const Real* v) {
+                                if (k >= nseed || nsurv + k >= ub) return;
+#pragma unroll
+                                for (int d = 0; d < DIM; ++d) {
+                                    w.xi[d][e0 + k] = xi[d];
+                                    w.v[d][e0 + k] = v[d];
+                                }
+                                w.perm[off - ob + nsurv + k] = (uint16_t)(e0 + k);
+                            });
+                        err |= sd.y;
+                        if (sd.x != nseed) err |= ERR_COUNT;
+                    }
+                    if (nsurv + nseed > ub) err |= ERR_COUNT_UB;
+                    write_holes(a, off + nsurv + nseed, off + ub, lane);
+                    if (lane == 0) new_range(a, c, off, ub);
+                }
+                __syncthreads();
+                for (uint32_t lc = cb + warp; lc < ce; lc += WT_WARPS) {
+                    const uint32_t c = c0 + lc, ub = w.off[lc + 1] - w.off[lc], nseed = w.sb[lc + 1] - w.sb[lc];
+                    const uint16_t* perm = w.perm + (w.off[lc] - ob);
+                    uint32_t ns;
+                    uint32_t fin = survivors_of(lc, ns) + nseed;
+                    fin = fin < ub ? fin : ub;
+                    if constexpr (HX) {
+                        const double s = partial_seq64<DIM, TCAP>(w.xi, w.v, fin, lane, [&](uint32_t r) { return (uint32_t)perm[r]; });
+                        if (lane < Dims<DIM>::PW) reinterpret_cast<double*>(a.partials)[(size_t)c * Dims<DIM>::PW + lane] = s;
+                    } else {
+                        PartialAcc<Real> acc;
+                        const uint32_t L = w.cs[lc + 1] - w.cs[lc], na = w.aoff[lc + 1] - w.aoff[lc];
+                        // no new particles, none removed by its counts alone (the cell's count exceeds its
+                        // occupied parts by at most max) and one round: rows are the old slots, then the
+                        // arrivals, with the leavers' rows empty
+                        if (nseed == 0 && L + na <= 32u &&
+                            (!apply || (maxpp >= 0 && ub <= w.occ[lc] + (uint32_t)maxpp))) {
+                            uint32_t e = 0;
+                            bool act = false;
+                            if ((uint32_t)lane < L) {
+                                e = w.cs[lc] - SA + lane;
+                                act = (w.mask[e >> 5] >> (e & 31u)) & 1u;
+                            } else if ((uint32_t)lane < L + na) {
+                                act = ns + lane - L < fin;
+                                e = act ? perm[ns + lane - L] : 0u;
+                            }
+                            Real xs[DIM], vs[DIM];
+#pragma unroll
+                            for (int d = 0; d < DIM; ++d) {
+                                xs[d] = w.xi[d][e];
+                                vs[d] = w.v[d][e];
+                            }
+                            partial_pairs32<DIM, false>(w.tr[warp], act, xs, vs, lane, acc);
+                        } else {
+                            for (uint32_t r0 = 0; r0 < fin; r0 += 32) {
+                                const bool act = r0 + lane < fin;
+                                const uint32_t e = act ? perm[r0 + lane] : 0u;
+                                Real xs[DIM], vs[DIM];
+#pragma unroll
+                                for (int d = 0; d < DIM; ++d) {
+                                    xs[d] = w.xi[d][e];
+                                    vs[d] = w.v[d][e];
+                                }
+                                __syncwarp();
+                                partial_pairs32<DIM, true>(w.tr[warp], act, xs, vs, lane, acc);
+                            }
+                        }
+                        __syncwarp();
+                        store_partial<DIM, Real>(a, c, acc, lane);
+                    }
+                }
+            }
+            cb = ce;
+            if (cb < ncell) __syncthreads();
+        }
+    }
+    warp_count(&a.stats->removed, removed);
+    warp_count(&a.stats->step_holes, removed);
+    err = __reduce_or_sync(0xffffffffu, err);
+    if (lane == 0 && err) atomicOr(&a.stats->error_flags, err);
+    // the last block to finish finalises the step (no waiting: the others
+    // have published their counters before counting themselves done)
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(&a.stats->write_done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            finalize_step(a);
+            a.stats->write_done = 0;
+            a.stats->write_next = 0;
+        }
+    }
+}
+
+}  // namespace pfem2
