@@ -59,10 +59,10 @@ __device__ __forceinline__ void interp_v(const void* Vc, uint32_t c, const Real*
 // A new particle at the centre of part idx of cell c (seed_particles
 // :87-104 and check_particle_distribution :390-407): xi = (idx + 1/2) h,
 // x = F(xi) (FP64 form), v = V interpolated at xi in FP64 (rounded to the
-// form's precision).  Returns xi and v.
+// form's precision).
 template <int DIM, typename Real>
-__device__ __forceinline__ void new_particle(const StepArgs& a, const PartState& S, uint32_t dst, uint32_t c,
-                                             const int* idx, uint32_t id, Real* xi, Real* v)
+__device__ __forceinline__ void new_particle_at(const StepArgs& a, uint32_t c, const int* idx, Real* xi, Real* v,
+                                                double* x)
 {
     double xid[DIM], vd[DIM];
 #pragma unroll
@@ -74,14 +74,23 @@ __device__ __forceinline__ void new_particle(const StepArgs& a, const PartState&
 #pragma unroll
     for (int d = 0; d < DIM; ++d) v[d] = (Real)vd[d];
     if constexpr (std::is_same<Real, double>::value) {
-        double X[1 << DIM][DIM], x[DIM];
+        double X[1 << DIM][DIM];
         load_cell64<DIM>(a.mesh.cellX, c, X);
         fwd64<DIM>(X, xid, x);
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) str<double>(S.x[d], dst, x[d]);
     }
+}
+
+// The same stored into slot dst of a state.
+template <int DIM, typename Real>
+__device__ __forceinline__ void new_particle(const StepArgs& a, const PartState& S, uint32_t dst, uint32_t c,
+                                             const int* idx, uint32_t id)
+{
+    Real xi[DIM], v[DIM];
+    double x[DIM];
+    new_particle_at<DIM, Real>(a, c, idx, xi, v, x);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
+        if constexpr (std::is_same<Real, double>::value) str<double>(S.x[d], dst, x[d]);
         str<Real>(S.xi[d], dst, xi[d]);
         str<Real>(S.v[d], dst, v[d]);
     }
@@ -118,8 +127,7 @@ __global__ void k_seed(StepArgs a, uint32_t* cell_start)
         const int k = (int)(t % a.pp.npart);
         int idx[3];
         part_digits<DIM>(k, a.pp, idx);
-        Real xi[DIM], v[DIM];
-        new_particle<DIM, Real>(a, a.S0, t, c, idx, id0 + t + 1, xi, v);
+        new_particle<DIM, Real>(a, a.S0, t, c, idx, id0 + t + 1);
         if (k == 0) cell_start[c] = t;
         if (a.chunk_first && t % ADV_CH == 0) a.chunk_first[t / ADV_CH] = c;
     }

@@ -91,8 +91,8 @@ template <int DIM>
 static int write32_t(const StepArgs& a, cudaStream_t s)
 {
     const int smem = (int)sizeof(WtTile<DIM, float>);
-    static const int grid = smem_grid32(k_write<DIM, float>, WT_THREADS, smem);
-    return launch_pdl(k_write<DIM, float>, grid, WT_THREADS, smem, s, a);
+    static const int grid = smem_grid32(k_write<DIM, float>, (WtCfg<DIM, float>::THREADS), smem);
+    return launch_pdl(k_write<DIM, float>, grid, (WtCfg<DIM, float>::THREADS), smem, s, a);
 }
 
 int launch_write(int dim, int prec, const StepArgs& a, cudaStream_t s)

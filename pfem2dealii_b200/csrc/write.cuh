@@ -11,13 +11,21 @@
 // takes the partial sums from the staged entries in the new order.
 //
 // What bounds it, and why tiles.  A time step's memory traffic here is 69
-// bytes a particle (FP32, 3D).  One warp per cell with one register round per
-// 32 particles (the layout before) lost its lanes to cells of 33 or 97
-// particles, could stage four cells only at seeding density, re-read the
-// written particles for the partial sums of cells above 32, and sent cells
-// above 96 to a path that counts positions through global scratch.  A run
-// settles near 1.9 particles per part (54 a cell at 27 parts, 124 at 64), so
-// those were the paths in use.
+// bytes a particle (FP32, 3D): 73 us for 7 M at the HBM rate.  One warp per
+// cell with one register round per 32 particles (the layout before) lost its
+// lanes to cells of 33 or 97 particles, could stage four cells only at
+// seeding density, re-read the written particles for the partial sums of
+// cells above 32, and sent cells above 96 to a path that counts positions
+// through global scratch.  A run settles near 1.9 particles per part (54 a
+// cell at 27 parts, 124 at 64), so those were the paths in use.  Measured,
+// before -> now: duct FP32 (7.0 M particles) 480 -> 199 us, FP64 940 -> 489;
+// cube FP32 (32 M) 8414 -> 917, 37^3 cube FP64 (6.2 M) 3253 -> 465; Turek
+// mesh FP32 (1.9 M) 291 -> 100, FP64 429 -> 162.  Now bound by instruction
+// issue and the latencies a tile waits on one after the other (its copies,
+// about a third of its time, five barriers): a tile's headers and first
+// arrivals are therefore copied while the tile before it is worked on, and
+// its new particles, whose parts are known from the move's occupancy, are
+// computed while its copies are in flight (221 -> 199 us with both).
 #pragma once
 
 #include "cellwork.cuh"
@@ -57,7 +65,7 @@ __device__ __forceinline__ void store_particle(const StepArgs& a, uint32_t dst, 
     }
 }
 
-// Empty slots [from, to) of a cell's range.
+// Empty slots [from, to) of a cell's range (one warp).
 __device__ __forceinline__ void write_holes(const StepArgs& a, uint32_t from, uint32_t to, int lane)
 {
     for (uint32_t j = from + lane; j < to; j += 32)
@@ -65,11 +73,11 @@ __device__ __forceinline__ void write_holes(const StepArgs& a, uint32_t from, ui
 }
 
 // New particles of one cell (one warp): the k-th seeded part (in part order)
-// goes to slot base + k and gets id id0 + sb + k + 1; stage(k, xi, v) sees it.
-// Returns the number of new particles and error bits.
-template <int DIM, typename Real, typename F>
+// goes to slot base + k and gets id id0 + sb + k + 1.  Returns the number of
+// new particles and error bits.
+template <int DIM, typename Real>
 __device__ __forceinline__ uint2 write_seeds(const StepArgs& a, uint32_t c, const int* cnt, uint32_t n, uint32_t base,
-                                             uint32_t id0, uint32_t sb, int lane, F&& stage)
+                                             uint32_t id0, uint32_t sb, int lane)
 {
     uint32_t done = 0, err = 0;
     for (int p0 = 0; p0 < a.pp.npe; p0 += 32) {
@@ -81,13 +89,8 @@ __device__ __forceinline__ uint2 write_seeds(const StepArgs& a, uint32_t c, cons
             const uint32_t dst = base + k;
             int idx[3] = {0, 0, 0};
             real_part<DIM>(p, a.pp, idx);
-            Real xi[DIM], v[DIM];
-            if (dst < a.capacity) {
-                new_particle<DIM, Real>(a, a.S1, dst, c, idx, id0 + sb + k + 1, xi, v);
-                stage(k, xi, v);
-            } else {
-                err |= ERR_CAPACITY;
-            }
+            if (dst < a.capacity) new_particle<DIM, Real>(a, a.S1, dst, c, idx, id0 + sb + k + 1);
+            else err |= ERR_CAPACITY;
         }
         done += __popc(m);
     }
@@ -187,8 +190,7 @@ __device__ __noinline__ uint2 write_cell_general(const StepArgs& a, int* cnt, Re
         load_global<DIM, Real>(a, g.x, pd);
         store_particle<DIM, Real>(a, off + pos, c, pd);
     }
-    const uint2 sd = write_seeds<DIM, Real>(a, c, cnt, n, off + nsurv, id0, sb, lane,
-                                            [](uint32_t, const Real*, const Real*) {});
+    const uint2 sd = write_seeds<DIM, Real>(a, c, cnt, n, off + nsurv, id0, sb, lane);
     err |= sd.y;
     const uint32_t nseed = sd.x;
     const uint32_t fin = nsurv + nseed;
@@ -292,73 +294,114 @@ __device__ __forceinline__ double partial_seq64(const double (*xi)[CAP], const d
                                                 At&& at)
 {
     const int iv = (lane >> 2) & ((1 << DIM) - 1), comp = lane & 3;
+    const double* vc = v[comp < DIM ? comp : 0];
     double acc = 0.0;
-    for (uint32_t r0 = 0; r0 < fin; r0 += 4) {
+    auto group = [&](uint32_t r0, uint32_t n) {
         const uint32_t own = at(r0 + comp < fin ? r0 + comp : r0);
         double N = lag64(iv & 1, xi[0][own]);
         N = N * lag64((iv >> 1) & 1, xi[1][own]);
         if (DIM > 2) N = N * lag64((iv >> 2) & 1, xi[DIM - 1][own]);
+        double t[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const double Nj = __shfl_sync(0xffffffffu, N, (lane & ~3) | j);
             const uint32_t e = __shfl_sync(0xffffffffu, own, (lane & ~3) | j);
-            if (r0 + j < fin) {
-                const double t = comp < DIM ? Nj * v[comp < DIM ? comp : 0][e] : (comp == DIM ? Nj : 0.0);
-                acc = acc + t;
-            }
+            t[j] = comp < DIM ? Nj * vc[e] : (comp == DIM ? Nj : 0.0);
         }
-    }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if ((uint32_t)j < n) acc = acc + t[j];
+    };
+    uint32_t r0 = 0;
+#pragma unroll 2
+    for (; r0 + 4 <= fin; r0 += 4) group(r0, 4);
+    if (r0 < fin) group(r0, fin - r0);
     return acc;
 }
 
+// Copies of a few bytes, global -> shared, that complete at async_wait.
+template <int BYTES>
+__device__ __forceinline__ void async_copy(void* dst, const void* src)
+{
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // Tiles.  TCAP entries (old slots, arrivals, new particles) fit one tile's
-// shared memory: 6 blocks of 128 threads per SM in the FP32 form, 4 in the
-// FP64 form.  The kernel takes as many cells per tile as bring it near TARGET
-// particles at the layout's mean density, fewer where the tiles would not
-// fill the grid; a tile that holds more than TCAP is worked through in runs
-// of cells that fit, and a single cell beyond TCAP takes the general path.
+// shared memory.  The kernel takes as many cells per tile as bring it near
+// TARGET particles at the layout's mean density, fewer where the tiles would
+// not fill the grid; a tile that holds more than TCAP is worked through in
+// runs of cells that fit, and a single cell beyond TCAP takes the general
+// path.  Sizes measured (write pass, us; FP32 duct of 7.0 M particles / cube
+// of 32 M): 512 entries, 7 blocks per SM 215 / 990; 640, 6 blocks 199 / 917;
+// 896, 5 blocks 202 / 868, which leaves smaller meshes too few tiles.  FP64
+// (duct / 37^3 cube): 384, 5 blocks 520 / 532; 512, 4 blocks 489 / 465.
 // ---------------------------------------------------------------------------
-constexpr int WT_WARPS = 4, WT_THREADS = WT_WARPS * 32;
 constexpr int WT_CELLS = 24;  // cells per tile at most
 constexpr int WT_CNT = 1024;  // part counters of a run of cells
+constexpr int WT_ARR = 8;     // arrivals per cell copied with its header
+constexpr int WT_OCC = 32;    // occupancy words of a tile: cells x ceil(npe / 64), where cells x npe <= WT_CNT
 
 template <int DIM, typename Real>
 struct WtCfg {
     static constexpr bool HX = std::is_same<Real, double>::value;
-    static constexpr int TCAP = HX ? 480 : 512;
-    static constexpr int TARGET = HX ? 440 : 470;
+    static constexpr int TCAP = HX ? 512 : 640;
+    static constexpr int TARGET = HX ? 470 : 600;
+    static constexpr int WARPS = 4, THREADS = WARPS * 32, BLOCKS = HX ? 4 : 6;
+};
+
+// What a tile needs to know of its cells, copied while the tile before it is
+// worked on.
+struct __align__(16) WtHead {
+    uint32_t arr[WT_CELLS][WT_ARR];  // the first arrivals
+    unsigned long long occ[WT_OCC];  // occupied parts, occw words per cell
+    uint2 co[WT_CELLS + 1];          // x: new slot offset, y: new particles before
+    uint32_t cs[WT_CELLS + 1];       // old slots
+    uint32_t na[WT_CELLS];           // arrivals
+    uint32_t aoff[WT_CELLS + 1];     // and their offsets in the tile
 };
 
 template <int DIM, typename Real>
 struct __align__(128) WtTile {
     static constexpr bool HX = WtCfg<DIM, Real>::HX;
     static constexpr int TCAP = WtCfg<DIM, Real>::TCAP;
-    uint32_t key[TCAP];  // the move's cell, then key_of(id)
-    uint32_t id[TCAP];
+    union {
+        struct {
+            uint32_t key[TCAP];  // old slots: the move's cell; arrivals: key_of(id)
+            uint32_t id[TCAP];
+            int cnt[WT_CNT];
+            uint16_t meta[TCAP];  // arrivals, new particles, over-full parts: local cell << 8 | extended part
+        };
+        Real tr[HX ? 1 : WtCfg<DIM, Real>::WARPS][HX ? 1 : 16][TRW];  // FP32 partial rows, 16 per warp (once placed)
+    };
     Real xi[DIM][TCAP];
     Real v[DIM][TCAP];
     Real x[HX ? DIM : 1][HX ? TCAP : 4];
-    Real tr[HX ? 1 : WT_WARPS][HX ? 1 : 16][TRW];  // FP32 partial rows, one block of 16 per warp
-    int cnt[WT_CNT];
-    uint16_t meta[TCAP];  // local cell << 8 | extended part; 0xffff: not in the new layout
-    uint16_t perm[TCAP];  // over-full parts' entries, then the entry of each new slot
-    uint32_t mask[TCAP / 32 + 1];  // survivors
-    uint32_t cs[WT_CELLS + 1], aoff[WT_CELLS + 1], off[WT_CELLS + 1], sb[WT_CELLS + 1];
-    uint32_t head[WT_CELLS], occ[WT_CELLS];
+    uint16_t perm[TCAP];       // over-full parts' entries, then the entry of each new slot
+    uint32_t mask[TCAP / 32];  // survivors
+    WtHead hdr[2];             // this tile's cells and the next one's
     uint64_t bar;
     uint32_t ticket, nover;
 };
 
 template <int DIM, typename Real>
-__global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ StepArgs a)
+__global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>::BLOCKS))
+    k_write(const __grid_constant__ StepArgs a)
 {
     constexpr bool HX = WtCfg<DIM, Real>::HX;
     constexpr int TCAP = WtCfg<DIM, Real>::TCAP, TARGET = WtCfg<DIM, Real>::TARGET;
-    static_assert(TCAP % 32 == 0 && TCAP / 32 < 32, "one survivor word per lane");
+    constexpr int WARPS = WtCfg<DIM, Real>::WARPS, THREADS = WARPS * 32, ROUNDS = TCAP / THREADS;
+    constexpr int HW = WARPS - 1;  // the warp that keeps the tickets and the headers
+    constexpr uint32_t NONE = 0xffffu;
+    static_assert(TCAP % THREADS == 0 && TCAP / 32 < 32, "whole rounds, one survivor word per lane");
     extern __shared__ __align__(128) unsigned char wr_raw[];
     auto& w = *reinterpret_cast<WtTile<DIM, Real>*>(wr_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const unsigned ltm = (1u << lane) - 1u;
     if (tid == 0) {
         mbar_init(&w.bar, 1);
         mbar_fence_init();
@@ -367,91 +410,103 @@ __global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ St
     pdl_entry();
     const uint32_t nC = (uint32_t)a.mesh.nC, cap = a.capacity;
     const uint32_t id0 = a.stats->next_id;
-    const int apply = a.apply_counts, maxpp = a.pp.maxpp, npe = a.pp.npe;
+    const int apply = a.apply_counts, maxpp = a.pp.maxpp, npe = a.pp.npe, occw = a.pp.occw;
     uint32_t NC;  // cells per tile
     {
-        const unsigned long long total = a.coff[nC] & 0xffffffffull;
+        // near TARGET particles at the mean density; in one wave of blocks, or in at least 8 (cells
+        // differ: on the Turek mesh 5 waves take 122 us, 8 take 100, 12 take 108), each wave full
+        const uint32_t total = (uint32_t)a.coff[nC];
         const unsigned long long by_load = total ? (unsigned long long)TARGET * nC / total : WT_CELLS;
-        const uint32_t by_grid = (nC + gridDim.x - 1) / gridDim.x, by_cnt = WT_CNT / npe;
+        const uint32_t by_cnt = WT_CNT / npe;
         NC = by_load < WT_CELLS ? (uint32_t)by_load : WT_CELLS;
-        NC = min(min(NC, by_grid), by_cnt);
+        NC = max(min(NC, by_cnt), 1u);
+        uint32_t waves = (nC + NC * gridDim.x - 1) / (NC * gridDim.x);
+        if (waves > 1 && waves < 8) waves = 8;
+        NC = min(NC, (nC + waves * gridDim.x - 1) / (waves * gridDim.x));
         NC = NC < 1 ? 1 : NC;
     }
     const uint32_t ntiles = (nC + NC - 1) / NC;
+    auto cells_of = [&](uint32_t tile) { return tile >= ntiles ? 0u : nC - tile * NC < NC ? nC - tile * NC : NC; };
     unsigned long long removed = 0;
     uint32_t err = 0, phase = 0;
     bool stage_ok = true;  // cleared for good if a copy ever fails to land in time
-    if (tid == 0) w.ticket = atomicAdd(&a.stats->write_next, 1u);
-    while (true) {
+    auto fetch_head = [&](WtHead& h, uint32_t tile) {
+        const uint32_t c0 = tile * NC, ncell = cells_of(tile);
+        if (ncell && (uint32_t)lane <= ncell) {
+            async_copy<4>(&h.cs[lane], a.cs_old + c0 + lane);
+            async_copy<8>(&h.co[lane], a.coff + c0 + lane);
+        }
+        if ((uint32_t)lane < ncell) {
+            async_copy<4>(&h.na[lane], a.carr + c0 + lane);
+#pragma unroll
+            for (int k = 0; k < WT_ARR; k += 4)
+                async_copy<16>(&h.arr[lane][k], a.carrs + (size_t)(c0 + lane) * ARRCAP + k);
+        }
+        if ((uint32_t)lane < ncell * occw) async_copy<8>(&h.occ[lane], a.cocc + (size_t)c0 * occw + lane);
+    };
+    auto land_head = [&](WtHead& h, uint32_t tile) {
+        async_wait();
+        __syncwarp();
+        const uint32_t ncell = cells_of(tile);
+        const uint32_t na = (uint32_t)lane < ncell ? h.na[lane] : 0u;
+        uint32_t inc = na;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if ((uint32_t)lane <= ncell) h.aoff[lane] = inc - na;
+        if (lane == 0) w.ticket = tile;
+    };
+    uint32_t tk = 0;  // (the header warp) the next tile
+    if (warp == HW) {
+        if (lane == 0) tk = atomicAdd(&a.stats->write_next, 2u);
+        tk = __shfl_sync(0xffffffffu, tk, 0);
+        fetch_head(w.hdr[0], tk);
+        land_head(w.hdr[0], tk);
+        ++tk;
+    }
+    for (uint32_t hb = 0;; hb ^= 1u) {
         __syncthreads();
         const uint32_t tile = w.ticket;
         if (tile >= ntiles) break;
-        const uint32_t c0 = tile * NC, ncell = nC - c0 < NC ? nC - c0 : NC;
-        uint32_t next_ticket = 0;
-        if (warp == 0) {  // the cells' headers, one cell per lane; their counters are reset for the next move
-            const bool in = (uint32_t)lane < ncell;
-            const uint32_t c = c0 + lane;
-            uint32_t na = 0;
-            if ((uint32_t)lane <= ncell) {
-                const unsigned long long o = a.coff[c];
-                w.cs[lane] = a.cs_old[c];
-                w.off[lane] = (uint32_t)o;
-                w.sb[lane] = (uint32_t)(o >> 32);
-            }
-            if (in) {
-                na = a.carr[c];
-                w.head[lane] = a.head[c];
-                uint32_t occ = 0;
-                for (int q = 0; q < a.pp.occw; ++q) {
-                    occ += __popcll(a.cocc[(size_t)c * a.pp.occw + q]);
-                    a.cocc[(size_t)c * a.pp.occw + q] = 0ull;
-                }
-                w.occ[lane] = occ;
-                a.carr[c] = 0;
-                a.ccount[c] = 0;
-                a.head[c] = LOST;
-            }
-            uint32_t inc = na;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += y;
-            }
-            if ((uint32_t)lane <= ncell) w.aoff[lane] = inc - na;
-            if (lane == 0) next_ticket = atomicAdd(&a.stats->write_next, 1u);
+        const uint32_t c0 = tile * NC, ncell = cells_of(tile);
+        const WtHead& h = w.hdr[hb];
+        uint32_t tk2 = 0;
+        if (warp == HW) {
+            fetch_head(w.hdr[hb ^ 1u], tk);
+            if (lane == 0) tk2 = atomicAdd(&a.stats->write_next, 1u);
         }
-        __syncthreads();
-        if (tid == 0) w.ticket = next_ticket;
         for (uint32_t cb = 0; cb < ncell;) {
             // the longest run of cells [cb, ce) that fits
-            const uint32_t SA = w.cs[cb] & ~3u;
+            const uint32_t SA = h.cs[cb] & ~3u, a0 = h.aoff[cb], ob = h.co[cb].x, sb0 = h.co[cb].y;
             uint32_t ce;
             {
                 const uint32_t j = cb + 1 + lane;
                 bool fits = false;
                 if (j <= ncell) {
-                    const uint32_t ent = ((w.cs[j] + 3u) & ~3u) - SA + (w.aoff[j] - w.aoff[cb]) + (w.sb[j] - w.sb[cb]);
-                    fits = ent <= (uint32_t)TCAP && w.off[j] - w.off[cb] <= (uint32_t)TCAP;
+                    const uint32_t ent = ((h.cs[j] + 3u) & ~3u) - SA + (h.aoff[j] - a0) + (h.co[j].y - sb0);
+                    fits = ent <= (uint32_t)TCAP && h.co[j].x - ob <= (uint32_t)TCAP;
                 }
                 ce = cb + (uint32_t)__popc(__ballot_sync(0xffffffffu, fits));
             }
             if (ce == cb) {  // a single cell beyond a tile
                 if (warp == 0) {
-                    const uint32_t c = c0 + cb, off = w.off[cb], ub = w.off[cb + 1] - off;
-                    // its rows live where a tile's entries would
-                    auto* tr = reinterpret_cast<Real(*)[TRW]>(HX ? (void*)&w.xi[0][0] : (void*)&w.tr[0][0][0]);
-                    const uint2 gr = write_cell_general<DIM, Real>(a, w.cnt, tr, c, w.cs[cb], w.cs[cb + 1] - w.cs[cb],
-                                                                   w.aoff[cb + 1] - w.aoff[cb], w.head[cb], off, ub,
-                                                                   w.sb[cb + 1] - w.sb[cb], w.sb[cb], id0, lane);
-                    if (lane == 0) new_range(a, c, off, ub);
+                    const uint32_t c = c0 + cb, ub = h.co[cb + 1].x - ob;
+                    auto* tr = reinterpret_cast<Real(*)[TRW]>(&w.xi[0][0]);  // rows where a tile's entries would be
+                    const uint2 gr =
+                        write_cell_general<DIM, Real>(a, w.cnt, tr, c, h.cs[cb], h.cs[cb + 1] - h.cs[cb], h.na[cb],
+                                                      a.head[c], ob, ub, h.co[cb + 1].y - sb0, sb0, id0, lane);
+                    if (lane == 0) new_range(a, c, ob, ub);
                     removed += gr.x;
                     err |= gr.y;
                 }
                 ce = cb + 1;
             } else {
-                const uint32_t E = w.cs[ce], EA = (E + 3u) & ~3u;
-                const uint32_t nold = w.cs[cb] < E ? EA - SA : 0u, a0 = w.aoff[cb], narr = w.aoff[ce] - a0;
-                const uint32_t nE = nold + narr, nch = (nE + 31u) >> 5;
+                // Entries: the old slots [SA, EA), the arrivals, the new particles.
+                const uint32_t E = h.cs[ce], EA = (E + 3u) & ~3u;
+                const uint32_t nold = h.cs[cb] < E ? EA - SA : 0u, narr = h.aoff[ce] - a0;
+                const uint32_t nE = nold + narr, nT = nE + (h.co[ce].y - sb0);
                 if (nold) {
                     if (stage_ok) {
                         if (tid == 0) {
@@ -471,7 +526,7 @@ __global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ St
                             }
                         }
                     } else {
-                        for (uint32_t j = tid; j < nold; j += WT_THREADS) {
+                        for (uint32_t j = tid; j < nold; j += THREADS) {
                             PData<DIM, Real> p;
                             load_global<DIM, Real>(a, SA + j, p);
                             w.key[j] = a.key[SA + j];
@@ -485,26 +540,29 @@ __global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ St
                         }
                     }
                 }
-                for (uint32_t t = tid; t < (ce - cb) * npe; t += WT_THREADS) w.cnt[t] = 0;
                 // arrivals beyond their cell's slots: one thread walks each overflow list
                 bool ovf = false;
-                if (cb + lane < ce) ovf = w.aoff[cb + lane + 1] - w.aoff[cb + lane] > (uint32_t)ARRCAP;
+                if (cb + lane < ce) ovf = h.na[cb + lane] > (uint32_t)ARRCAP;
                 if (__any_sync(0xffffffffu, ovf)) {
                     if (warp == 0 && ovf) {
-                        const uint32_t lc = cb + lane, na = w.aoff[lc + 1] - w.aoff[lc];
-                        uint32_t p = w.head[lc];
+                        const uint32_t lc = cb + lane, na = h.na[lc];
+                        uint32_t p = a.head[c0 + lc];
                         for (uint32_t k = ARRCAP; k < na; ++k) {
-                            w.key[nold + (w.aoff[lc] - a0) + k] = p;
+                            w.key[nold + (h.aoff[lc] - a0) + k] = p;
                             if (p < cap) p = a.next[p];
                         }
                     }
                     __syncthreads();
                 }
-                for (uint32_t t = tid; t < narr; t += WT_THREADS) {
+                for (uint32_t t = tid; t < narr; t += THREADS) {
                     uint32_t lc = cb;
-                    while (w.aoff[lc + 1] - a0 <= t) ++lc;
-                    const uint32_t k = t - (w.aoff[lc] - a0), e = nold + t;
-                    const uint32_t i = k < (uint32_t)ARRCAP ? a.carrs[(size_t)(c0 + lc) * ARRCAP + k] : w.key[e];
+#pragma unroll
+                    for (uint32_t st = 16; st; st >>= 1)
+                        if (lc + st < ce && h.aoff[lc + st] - a0 <= t) lc += st;
+                    const uint32_t k = t - (h.aoff[lc] - a0), e = nold + t;
+                    const uint32_t i = k < (uint32_t)WT_ARR   ? h.arr[lc][k]
+                                       : k < (uint32_t)ARRCAP ? a.carrs[(size_t)(c0 + lc) * ARRCAP + k]
+                                                              : w.key[e];
                     if (i < cap) {
                         PData<DIM, Real> p;
                         load_global<DIM, Real>(a, i, p);
@@ -518,14 +576,51 @@ __global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ St
                         w.meta[e] = (uint16_t)(lc << 8);
                     } else {
                         err |= ERR_ARRIVAL;
-                        w.meta[e] = 0xffffu;
+                        w.meta[e] = (uint16_t)NONE;
                     }
                 }
+                for (uint32_t t = tid; t < (ce - cb) * npe; t += THREADS) w.cnt[t] = 0;
+                // new particles, while the copies are in flight: the real parts the move left empty
+                {
+                    uint32_t todo = __ballot_sync(0xffffffffu, cb + lane < ce && h.co[cb + lane + 1].y != h.co[cb + lane].y);
+                    for (int k = 1; todo; ++k, todo &= todo - 1) {
+                        if (k % WARPS != warp) continue;  // one cell per warp in turn, from the second warp on
+                        const uint32_t lc = cb + __ffs(todo) - 1, sb = h.co[lc].y, n1 = h.co[lc + 1].y - sb;
+                        uint32_t done = 0;
+                        for (int p0 = 0; p0 < npe; p0 += 32) {
+                            const int p = p0 + lane;
+                            const bool sf = p < npe && ((a.pp.realmask[p >> 6] >> (p & 63)) & 1ull) &&
+                                            (maxpp < 0 || !((h.occ[lc * occw + (p >> 6)] >> (p & 63)) & 1ull));
+                            const unsigned b = __ballot_sync(0xffffffffu, sf);
+                            const uint32_t j = done + __popc(b & ltm);
+                            if (sf && j < n1) {
+                                const uint32_t e = nE + (sb - sb0) + j;
+                                int idx[3] = {0, 0, 0};
+                                real_part<DIM>(p, a.pp, idx);
+                                Real xi[DIM], v[DIM];
+                                double x[DIM];
+                                new_particle_at<DIM, Real>(a, c0 + lc, idx, xi, v, x);
+#pragma unroll
+                                for (int d = 0; d < DIM; ++d) {
+                                    w.xi[d][e] = xi[d];
+                                    w.v[d][e] = v[d];
+                                    if constexpr (HX) w.x[d][e] = x[d];
+                                }
+                                w.id[e] = id0 + sb + j + 1;
+                                w.meta[e] = (uint16_t)(lc << 8);
+                            }
+                            done += __popc(b);
+                        }
+                        if (done != n1) err |= ERR_COUNT;
+                    }
+                }
+                async_wait();
                 if (nold && stage_ok) {
-                    if (__syncthreads_or(!mbar_wait(&w.bar, phase))) {
+                    // one thread polls, the others rest at the barrier
+                    if (__syncthreads_or(tid == 0 && !mbar_wait(&w.bar, phase))) {
                         // give the copy one more bounded wait, then stop staging; this run's particles are lost
                         err |= ERR_TIMEOUT;
-                        mbar_wait(&w.bar, phase);
+                        if (tid == 0) mbar_wait(&w.bar, phase);
                         stage_ok = false;
                         __syncthreads();
                     }
@@ -533,48 +628,53 @@ __global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ St
                 } else {
                     __syncthreads();
                 }
-                // cell, part and key of every entry; part counts
-                for (uint32_t e = tid; e < nE; e += WT_THREADS) {
-                    uint32_t m = 0xffffu;
+                // cell and part of every entry; part counts.  Entry r * THREADS + tid stays in this thread's
+                // registers; word r * WARPS + warp of the survivors is this warp's.
+                uint32_t m[ROUNDS];
+#pragma unroll
+                for (int r = 0; r < ROUNDS; ++r) {
+                    const uint32_t e = r * THREADS + tid;
+                    m[r] = NONE;
                     if (e < nold) {
                         const uint32_t lc = w.key[e] - c0, slot = SA + e;
-                        if (lc >= cb && lc < ce && slot >= w.cs[lc] && slot < w.cs[lc + 1]) m = lc << 8;
-                    } else {
-                        m = w.meta[e];
+                        if (lc >= cb && lc < ce && slot >= h.cs[lc] && slot < h.cs[lc + 1]) m[r] = lc << 8;
+                    } else if (e < nT) {
+                        m[r] = w.meta[e];
+                        if (e < nE) w.key[e] = key_of(w.id[e], a.pp.seed);
                     }
-                    if (m != 0xffffu) {
+                    if (e < nE && m[r] != NONE) {
                         Real xi[DIM];
 #pragma unroll
                         for (int d = 0; d < DIM; ++d) xi[d] = w.xi[d][e];
                         const int pe = ext_part<DIM, Real>(xi, a.pp);
-                        if (apply) atomicAdd(w.cnt + ((m >> 8) - cb) * npe + pe, 1);
-                        m |= (uint32_t)pe;
-                        w.key[e] = key_of(w.id[e], a.pp.seed);
+                        if (apply) atomicAdd(w.cnt + ((m[r] >> 8) - cb) * npe + pe, 1);
+                        m[r] |= (uint32_t)pe;
                     }
-                    w.meta[e] = (uint16_t)m;
                 }
                 __syncthreads();
                 // survivors: everyone outside the over-full parts, and there the smallest keys
                 bool over = false;
-                for (uint32_t e = tid; e < nch * 32u; e += WT_THREADS) {
-                    const uint32_t m = e < nE ? w.meta[e] : 0xffffu;
-                    bool live = m != 0xffffu;
-                    if (live && apply && w.cnt[((m >> 8) - cb) * npe + (m & 255u)] > maxpp + 1) {
+#pragma unroll
+                for (int r = 0; r < ROUNDS; ++r) {
+                    const uint32_t e = r * THREADS + tid;
+                    bool live = e < nE && m[r] != NONE;
+                    if (live && apply && w.cnt[((m[r] >> 8) - cb) * npe + (m[r] & 255u)] > maxpp + 1) {
                         w.perm[atomicAdd(&w.nover, 1u)] = (uint16_t)e;
+                        w.meta[e] = (uint16_t)m[r];
                         over = true;
                         live = false;
                     }
                     const unsigned b = __ballot_sync(0xffffffffu, live);
-                    if (lane == 0) w.mask[e >> 5] = b;
+                    if (lane == 0) w.mask[r * WARPS + warp] = b;
                 }
                 if (__syncthreads_or(over)) {
                     const uint32_t nov = w.nover;
-                    for (uint32_t j = tid; j < nov; j += WT_THREADS) {
-                        const uint32_t e = w.perm[j], m = w.meta[e], kk = w.key[e];
+                    for (uint32_t j = tid; j < nov; j += THREADS) {
+                        const uint32_t e = w.perm[j], me = w.meta[e], kk = key_of(w.id[e], a.pp.seed);
                         int rank = 0;
                         for (uint32_t o = 0; o < nov; ++o) {
                             const uint32_t f = w.perm[o];
-                            rank += (w.meta[f] == m && w.key[f] < kk) ? 1 : 0;
+                            rank += (w.meta[f] == me && key_of(w.id[f], a.pp.seed) < kk) ? 1 : 0;
                         }
                         if (rank < maxpp + 1) atomicOr(w.mask + (e >> 5), 1u << (e & 31u));
                         else removed++;
@@ -583,7 +683,7 @@ __global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ St
                     if (tid == 0) w.nover = 0;
                 }
                 // survivors before an entry: words by a scan over the lanes, bits by a count
-                const uint32_t word = (uint32_t)lane < nch ? w.mask[lane] : 0u;
+                const uint32_t word = lane < TCAP / 32 ? w.mask[lane] : 0u;
                 uint32_t wpre = __popc(word);
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
@@ -596,27 +696,41 @@ __global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ St
                     const uint32_t b = __shfl_sync(0xffffffffu, word, (int)(e >> 5));
                     return p + (uint32_t)__popc(b & ((1u << (e & 31u)) - 1u));
                 };
+                // the run's cells, one per lane: survivors before the cell's old slots, its stayers, all its survivors
+                uint32_t c_pb, c_ns, c_nsurv;
+                {
+                    const uint32_t lc = cb + lane < ce ? cb + lane : cb;
+                    c_pb = before(nold ? h.cs[lc] - SA : 0u);
+                    c_ns = before(nold ? h.cs[lc + 1] - SA : 0u) - c_pb;
+                    c_nsurv = c_ns + before(nold + h.aoff[lc + 1] - a0) - before(nold + h.aoff[lc] - a0);
+                }
                 // places and stores
-                const uint32_t ob = w.off[cb];
-                for (uint32_t e = tid; e < nch * 32u; e += WT_THREADS) {
-                    const uint32_t m = e < nE ? w.meta[e] : 0xffffu;
-                    const bool live = (w.mask[e >> 5] >> lane) & 1u;
-                    const uint32_t lc = live ? m >> 8 : cb;
-                    const uint32_t lb = nold ? w.cs[lc] - SA : 0u, le = nold ? w.cs[lc + 1] - SA : 0u;
-                    const uint32_t pb = before(lb), pe = before(le), ps = before(e);
+#pragma unroll
+                for (int r = 0; r < ROUNDS; ++r) {
+                    const uint32_t e = r * THREADS + tid;
+                    const uint32_t wd = __shfl_sync(0xffffffffu, word, r * WARPS + warp);
+                    const uint32_t ps = __shfl_sync(0xffffffffu, wpre, r * WARPS + warp) + __popc(wd & ltm);
+                    const bool live = ((wd >> lane) & 1u) || (e >= nE && e < nT);
+                    const uint32_t lc = live ? m[r] >> 8 : cb;
+                    const uint32_t pb = __shfl_sync(0xffffffffu, c_pb, (int)(lc - cb));
+                    const uint32_t nst = __shfl_sync(0xffffffffu, c_ns, (int)(lc - cb));
+                    const uint32_t nsv = __shfl_sync(0xffffffffu, c_nsurv, (int)(lc - cb));
                     if (!live) continue;
+                    const uint2 co = h.co[lc];
                     uint32_t pos;
                     if (e < nold) {
                         pos = ps - pb;
-                    } else {
-                        pos = pe - pb;
+                    } else if (e < nE) {  // arrivals by key
+                        pos = nst;
                         const uint32_t kk = w.key[e];
-                        const uint32_t o1 = nold + w.aoff[lc + 1] - a0;
-                        for (uint32_t o = nold + w.aoff[lc] - a0; o < o1; ++o)
+                        const uint32_t o1 = nold + h.aoff[lc + 1] - a0;
+                        for (uint32_t o = nold + h.aoff[lc] - a0; o < o1; ++o)
                             pos += (((w.mask[o >> 5] >> (o & 31u)) & 1u) && w.key[o] < kk) ? 1u : 0u;
+                    } else {
+                        pos = nsv + (e - nE - (co.y - sb0));
                     }
-                    const uint32_t dst = w.off[lc] + pos;
-                    if (pos >= w.off[lc + 1] - w.off[lc]) {
+                    const uint32_t dst = co.x + pos;
+                    if (pos >= h.co[lc + 1].x - co.x) {
                         err |= ERR_COUNT_UB;
                         continue;
                     }
@@ -634,60 +748,43 @@ __global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ St
                         if constexpr (HX) str<double>(a.S1.x[d], dst, w.x[d][e]);
                     }
                 }
-                // the cells' survivors, new particles and empty slots: a warp per cell, the same warp
-                // as for the sums below
-                auto survivors_of = [&](uint32_t lc, uint32_t& ns) {
-                    const uint32_t lb = nold ? w.cs[lc] - SA : 0u, le = nold ? w.cs[lc + 1] - SA : 0u;
-                    ns = before(le) - before(lb);
-                    return ns + before(nold + w.aoff[lc + 1] - a0) - before(nold + w.aoff[lc] - a0);
-                };
-                for (uint32_t lc = cb + warp; lc < ce; lc += WT_WARPS) {
-                    const uint32_t c = c0 + lc, off = w.off[lc], ub = w.off[lc + 1] - off;
-                    const uint32_t nseed = w.sb[lc + 1] - w.sb[lc];
-                    uint32_t ns;
-                    const uint32_t nsurv = survivors_of(lc, ns);
-                    if (nseed) {
-                        const uint32_t e0 = nE + (w.sb[lc] - w.sb[cb]);
-                        const uint2 sd = write_seeds<DIM, Real>(
-                            a, c, w.cnt + (lc - cb) * npe, 1u, off + nsurv, id0, w.sb[lc], lane,
-                            [&](uint32_t k, const Real* xi, const Real* v) {
-                                if (k >= nseed || nsurv + k >= ub) return;
-#pragma unroll
-                                for (int d = 0; d < DIM; ++d) {
-                                    w.xi[d][e0 + k] = xi[d];
-                                    w.v[d][e0 + k] = v[d];
-                                }
-                                w.perm[off - ob + nsurv + k] = (uint16_t)(e0 + k);
-                            });
-                        err |= sd.y;
-                        if (sd.x != nseed) err |= ERR_COUNT;
-                    }
-                    if (nsurv + nseed > ub) err |= ERR_COUNT_UB;
-                    write_holes(a, off + nsurv + nseed, off + ub, lane);
-                    if (lane == 0) new_range(a, c, off, ub);
+                // empty slots and the new ranges, a cell per lane
+                if (warp == HW && cb + lane < ce) {
+                    const uint2 co = h.co[cb + lane], cn = h.co[cb + lane + 1];
+                    for (uint32_t j = co.x + c_nsurv + (cn.y - co.y); j < cn.x; ++j)
+                        if (j < cap) a.S1.cell[j] = HOLE;
+                    new_range(a, c0 + cb + lane, co.x, cn.x - co.x);
                 }
                 __syncthreads();
-                for (uint32_t lc = cb + warp; lc < ce; lc += WT_WARPS) {
-                    const uint32_t c = c0 + lc, ub = w.off[lc + 1] - w.off[lc], nseed = w.sb[lc + 1] - w.sb[lc];
-                    const uint16_t* perm = w.perm + (w.off[lc] - ob);
-                    uint32_t ns;
-                    uint32_t fin = survivors_of(lc, ns) + nseed;
+                // partial sums, a warp per cell
+                for (uint32_t lc = cb + warp; lc < ce; lc += WARPS) {
+                    const uint32_t c = c0 + lc, ub = h.co[lc + 1].x - h.co[lc].x, nseed = h.co[lc + 1].y - h.co[lc].y;
+                    const uint16_t* perm = w.perm + (h.co[lc].x - ob);
+                    const uint32_t ns = __shfl_sync(0xffffffffu, c_ns, (int)(lc - cb));
+                    uint32_t fin = __shfl_sync(0xffffffffu, c_nsurv, (int)(lc - cb)) + nseed;
                     fin = fin < ub ? fin : ub;
                     if constexpr (HX) {
-                        const double s = partial_seq64<DIM, TCAP>(w.xi, w.v, fin, lane, [&](uint32_t r) { return (uint32_t)perm[r]; });
-                        if (lane < Dims<DIM>::PW) reinterpret_cast<double*>(a.partials)[(size_t)c * Dims<DIM>::PW + lane] = s;
+                        const double s = partial_seq64<DIM, TCAP>(w.xi, w.v, fin, lane,
+                                                                  [&](uint32_t r) { return (uint32_t)perm[r]; });
+                        if (lane < Dims<DIM>::PW)
+                            reinterpret_cast<double*>(a.partials)[(size_t)c * Dims<DIM>::PW + lane] = s;
                     } else {
                         PartialAcc<Real> acc;
-                        const uint32_t L = w.cs[lc + 1] - w.cs[lc], na = w.aoff[lc + 1] - w.aoff[lc];
+                        const uint32_t L = h.cs[lc + 1] - h.cs[lc], na = h.na[lc];
                         // no new particles, none removed by its counts alone (the cell's count exceeds its
                         // occupied parts by at most max) and one round: rows are the old slots, then the
                         // arrivals, with the leavers' rows empty
-                        if (nseed == 0 && L + na <= 32u &&
-                            (!apply || (maxpp >= 0 && ub <= w.occ[lc] + (uint32_t)maxpp))) {
+                        bool simple = nseed == 0 && L + na <= 32u;
+                        if (simple && apply) {
+                            uint32_t occ = 0;
+                            for (int q = 0; q < occw; ++q) occ += __popcll(h.occ[lc * occw + q]);
+                            simple = maxpp >= 0 && ub <= occ + (uint32_t)maxpp;
+                        }
+                        if (simple) {
                             uint32_t e = 0;
                             bool act = false;
                             if ((uint32_t)lane < L) {
-                                e = w.cs[lc] - SA + lane;
+                                e = h.cs[lc] - SA + lane;
                                 act = (w.mask[e >> 5] >> (e & 31u)) & 1u;
                             } else if ((uint32_t)lane < L + na) {
                                 act = ns + lane - L < fin;
@@ -703,7 +800,7 @@ __global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ St
                         } else {
                             for (uint32_t r0 = 0; r0 < fin; r0 += 32) {
                                 const bool act = r0 + lane < fin;
-                                const uint32_t e = act ? perm[r0 + lane] : 0u;
+                                const uint32_t e = perm[act ? r0 + lane : r0];
                                 Real xs[DIM], vs[DIM];
 #pragma unroll
                                 for (int d = 0; d < DIM; ++d) {
@@ -721,6 +818,18 @@ __global__ void __launch_bounds__(WT_THREADS) k_write(const __grid_constant__ St
             }
             cb = ce;
             if (cb < ncell) __syncthreads();
+        }
+        // the cells' counters, for the next move
+        if (warp == 0 && (uint32_t)lane < ncell) {
+            const uint32_t c = c0 + lane, na = h.na[lane];
+            a.ccount[c] = 0;
+            if (na) a.carr[c] = 0;
+            if (na > (uint32_t)ARRCAP) a.head[c] = LOST;
+            for (int q = 0; q < occw; ++q) a.cocc[(size_t)c * occw + q] = 0ull;
+        }
+        if (warp == HW) {
+            land_head(w.hdr[hb ^ 1u], tk);
+            tk = __shfl_sync(0xffffffffu, tk2, 0);
         }
     }
     warp_count(&a.stats->removed, removed);
