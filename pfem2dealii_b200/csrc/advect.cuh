@@ -34,6 +34,58 @@ struct SearchOut {
     uint32_t map_failures;
 };
 
+// inverse_map64 of cell c, out of line: for the points that locate_lin64
+// leaves undecided (within 1e-9 of a face, or far outside).
+template <int DIM>
+struct InvOut {
+    double xi[DIM];
+    int st;
+};
+template <int DIM>
+__device__ __noinline__ InvOut<DIM> inverse_full64(const double* cellX, const double* aff, uint32_t c, Vec<DIM> p)
+{
+    double X[1 << DIM][DIM];
+    load_cell64<DIM>(cellX, c, X);
+    InvOut<DIM> o;
+    o.st = inverse_map64<DIM>(X, aff + (size_t)c * Dims<DIM>::AFF, p.v, o.xi);
+    return o;
+}
+
+// inverse_map64's status, and its point where that lies inside the unit cell
+// (else some point outside it), for a mesh whose cells are safe for
+// locate_lin64.
+template <int DIM, typename Aff>
+__device__ __forceinline__ int inverse_lin64(const MeshDev& m, Aff&& aff, uint32_t c, const double* p, double* xi)
+{
+    if constexpr (DIM == 3) {
+        if (locate_lin64(aff, p, xi) < 2) return 0;
+    }
+    Vec<DIM> q;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) q.v[d] = p[d];
+    const InvOut<DIM> o = inverse_full64<DIM>(m.cellX, m.aff, c, q);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) xi[d] = o.xi[d];
+    return o.st;
+}
+
+// Inverse map of a candidate cell.  LIN: its exact affine inverse; FAST: the
+// Newton restatement's decision by inverse_lin64; else that restatement.
+template <int DIM, bool LIN, bool FAST>
+__device__ __forceinline__ int candidate64(const MeshDev& m, uint32_t cand, const double* p, double* xi)
+{
+    if constexpr (LIN) {
+        return inverse_affine64<DIM>(m.aff + (size_t)cand * Dims<DIM>::AFF, p, xi);
+    } else if constexpr (FAST) {
+        const double* ca = m.aff + (size_t)cand * Dims<DIM>::AFF;
+        return inverse_lin64<DIM>(m, [=](int j) { return __ldg(ca + j); }, cand, p, xi);
+    } else {
+        double X[1 << DIM][DIM];
+        load_cell64<DIM>(m.cellX, cand, X);
+        return inverse_map64<DIM>(X, m.aff + (size_t)cand * Dims<DIM>::AFF, p, xi);
+    }
+}
+
 // Vertex-patch search for a particle that left cell c
 // (sort_particles_into_subdomains_and_cells, src/pfem2particlehandler.cpp:438-491):
 //  1. closest vertex of c seen from the previous position F(xi_old) along
@@ -50,11 +102,10 @@ struct SearchOut {
 // candidate is the cell's exact affine inverse xi = A^-1 (p - b), one
 // matrix-vector product instead of the Newton iteration; the FP64 form
 // always takes the Newton restatement (bit parity with its CPU restatement).
-template <int DIM, bool LIN = false>
+template <int DIM, bool LIN = false, bool FAST = false>
 __device__ __noinline__ SearchOut search64(const MeshDev m, uint32_t c, Vec<DIM> xo, Vec<DIM> ve, Vec<DIM> xp)
 {
     constexpr int NV = 1 << DIM;
-    constexpr int AFF = Dims<DIM>::AFF;
     SearchOut out;
     out.cell = c;
     out.flags = 0;
@@ -102,59 +153,59 @@ __device__ __noinline__ SearchOut search64(const MeshDev m, uint32_t c, Vec<DIM>
         out.flags |= SRCH_OVERFLOW;
         n = MAX_CAND;
     }
-    if constexpr (LIN) {
-        // Up to REG_CAND candidates stay in registers: the next one tried is
-        // the untried maximum of the dot products, the first of equal ones
-        // (the order of the stable descending sort below), selected only
-        // when the ones before it have failed.
-        if (n <= REG_CAND) {
-            double dk[REG_CAND];
-            uint32_t ck[REG_CAND];
+    // Up to REG_CAND candidates stay in registers: the next one tried is the
+    // untried maximum of the dot products, the first of equal ones (the order
+    // of the stable descending sort below), selected only when the ones
+    // before it have failed.  (2D: the sort is the faster, 96 against 101 us
+    // for 412 k searches on the Turek mesh.)
+    if ((LIN || DIM == 3) && n <= REG_CAND) {
+        double dk[REG_CAND];
+        uint32_t ck[REG_CAND];
+#pragma unroll
+        for (int k = 0; k < REG_CAND; ++k) {
+            dk[k] = 0.0;
+            ck[k] = c;
+            if (k < n) {
+                const double* cd = m.v2c_dirs + (size_t)(b + k) * DIM;
+                double s = __ldg(cd) * vtp[0];
+#pragma unroll
+                for (int d = 1; d < DIM; ++d) s = s + __ldg(cd + d) * vtp[d];
+                dk[k] = s;
+                ck[k] = (uint32_t)__ldg(m.v2c_cells + b + k);
+            }
+        }
+        uint32_t tried = 0;
+        for (int t = 0; t < n; ++t) {
+            int bi = -1;
+            double bv = 0.0;
+            uint32_t cand = c;
 #pragma unroll
             for (int k = 0; k < REG_CAND; ++k) {
-                dk[k] = 0.0;
-                ck[k] = c;
-                if (k < n) {
-                    const double* cd = m.v2c_dirs + (size_t)(b + k) * DIM;
-                    double s = __ldg(cd) * vtp[0];
-#pragma unroll
-                    for (int d = 1; d < DIM; ++d) s = s + __ldg(cd + d) * vtp[d];
-                    dk[k] = s;
-                    ck[k] = (uint32_t)__ldg(m.v2c_cells + b + k);
+                const bool open = k < n && !((tried >> k) & 1u);
+                if (open && (bi < 0 || dk[k] > bv)) {
+                    bi = k;
+                    bv = dk[k];
+                    cand = ck[k];
                 }
             }
-            uint32_t tried = 0;
-            for (int t = 0; t < n; ++t) {
-                int bi = -1;
-                double bv = 0.0;
-                uint32_t cand = c;
-#pragma unroll
-                for (int k = 0; k < REG_CAND; ++k) {
-                    const bool open = k < n && !((tried >> k) & 1u);
-                    if (open && (bi < 0 || dk[k] > bv)) {
-                        bi = k;
-                        bv = dk[k];
-                        cand = ck[k];
-                    }
-                }
-                tried |= 1u << bi;
-                if (cand == c) continue;
-                double xin[DIM];
-                if (inverse_affine64<DIM>(m.aff + (size_t)cand * AFF, xp.v, xin)) {
-                    out.map_failures++;
-                    continue;
-                }
-                if (inside_unit<DIM>(xin)) {
-                    out.cell = cand;
-                    out.flags |= SRCH_FOUND;
-#pragma unroll
-                    for (int d = 0; d < DIM; ++d) out.xi[d] = xin[d];
-                    if (near_face64<DIM>(xin)) out.flags |= SRCH_NEAR;
-                    return out;
-                }
+            tried |= 1u << bi;
+            if (cand == c) continue;
+            double xin[DIM];
+            const int st = candidate64<DIM, LIN, FAST>(m, cand, xp.v, xin);
+            if (st) {
+                out.map_failures++;
+                continue;
             }
-            return out;
+            if (inside_unit<DIM>(xin)) {
+                out.cell = cand;
+                out.flags |= SRCH_FOUND;
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) out.xi[d] = xin[d];
+                if (near_face64<DIM>(xin)) out.flags |= SRCH_NEAR;
+                return out;
+            }
         }
+        return out;
     }
     double dots[MAX_CAND];
     uint8_t perm[MAX_CAND];
@@ -180,13 +231,7 @@ __device__ __noinline__ SearchOut search64(const MeshDev m, uint32_t c, Vec<DIM>
         const uint32_t cand = (uint32_t)__ldg(m.v2c_cells + b + perm[k]);
         if (cand == c) continue;
         double xin[DIM];
-        int st;
-        if constexpr (LIN) {
-            st = inverse_affine64<DIM>(m.aff + (size_t)cand * AFF, xp.v, xin);
-        } else {
-            load_cell64<DIM>(m.cellX, cand, X);
-            st = inverse_map64<DIM>(X, m.aff + (size_t)cand * AFF, xp.v, xin);
-        }
+        const int st = candidate64<DIM, LIN, FAST>(m, cand, xp.v, xin);
         if (st) {
             out.map_failures++;
             continue;
@@ -444,6 +489,34 @@ struct AdvRecStage {
     float4 v[MAXC][F4];
     float4 dv[MAXC][F4];
     uint32_t cfirst, ncell;
+    __device__ static uint32_t bytes(const StepArgs& a, uint32_t n) { return n * F4 * 16u * (a.do_correct ? 2u : 1u); }
+    __device__ void issue(const StepArgs& a, uint32_t cf, uint32_t n, uint64_t* bar)
+    {
+        bulk_g2s(v, a.vrec32 + (size_t)cf * F4 * 4, n * F4 * 16u, bar);
+        if (a.do_correct) bulk_g2s(dv, a.dvrec32 + (size_t)cf * F4 * 4, n * F4 * 16u, bar);
+    }
+};
+
+// FP64 form on meshes safe for locate_lin64: the vertex velocities (V and
+// V - Vold) and the affine inverses of the chunk's cells.  The loads of these
+// (24 + 24 + 12 doubles a particle, the first 24 in every sub-step) from
+// global memory held every warp for 4 of its 11 cycles per instruction.
+struct __align__(16) AdvLin64Stage {
+    static constexpr int MAXC = 24, VW = 32, AW = 12;
+    double v[MAXC][VW];
+    double dv[MAXC][VW];
+    double aff[MAXC][AW];
+    uint32_t cfirst, ncell;
+    __device__ static uint32_t bytes(const StepArgs& a, uint32_t n)
+    {
+        return n * 8u * (VW * (a.do_correct ? 2u : 1u) + AW);
+    }
+    __device__ void issue(const StepArgs& a, uint32_t cf, uint32_t n, uint64_t* bar)
+    {
+        bulk_g2s(v, reinterpret_cast<const double*>(a.Vc) + (size_t)cf * VW, n * VW * 8u, bar);
+        if (a.do_correct) bulk_g2s(dv, reinterpret_cast<const double*>(a.dVc) + (size_t)cf * VW, n * VW * 8u, bar);
+        bulk_g2s(aff, a.mesh.aff + (size_t)cf * AW, n * AW * 8u, bar);
+    }
 };
 
 // A chunk ticket and, for the record stage, the chunk's first and last
@@ -471,9 +544,9 @@ __device__ __forceinline__ void ticket_cells(const StepArgs& a, uint32_t n, Chun
 // st, and (rs not null) the records of the chunk's cells [t.cf, t.cl] into
 // rs (a range that is out of order or too long is not staged; the particles
 // then read their records from global memory).
-template <int DIM, typename Real, int CH>
+template <int DIM, typename Real, int CH, typename RS>
 __device__ __forceinline__ void stage_chunk(const StepArgs& a, AdvStage<DIM, Real, CH>& st, uint64_t* bar,
-                                            const ChunkTicket& t, uint32_t n, AdvRecStage<DIM>* rs = nullptr)
+                                            const ChunkTicket& t, uint32_t n, RS* rs)
 {
     constexpr bool HX = std::is_same<Real, double>::value;
     const uint32_t chunk = t.tk;
@@ -484,17 +557,12 @@ __device__ __forceinline__ void stage_chunk(const StepArgs& a, AdvStage<DIM, Rea
     if (rs) {
         const uint32_t nC = (uint32_t)a.mesh.nC;
         cf = t.cf;
-        if (t.cf <= t.cl && t.cl < nC && t.cl - t.cf < (uint32_t)AdvRecStage<DIM>::MAXC) nrec = t.cl - t.cf + 1;
+        if (t.cf <= t.cl && t.cl < nC && t.cl - t.cf < (uint32_t)RS::MAXC) nrec = t.cl - t.cf + 1;
         rs->cfirst = cf;
         rs->ncell = nrec;
     }
-    constexpr uint32_t RB = Dims<DIM>::REC4 * 16u;  // bytes of one cell's record
-    const uint32_t recb = nrec * RB * (a.do_correct ? 2u : 1u);
-    mbar_expect_tx(bar, b4 + (2 + (HX ? 1 : 0)) * DIM * br + recb);
-    if (nrec) {
-        bulk_g2s(rs->v, a.vrec32 + (size_t)cf * Dims<DIM>::REC4 * 4, nrec * RB, bar);
-        if (a.do_correct) bulk_g2s(rs->dv, a.dvrec32 + (size_t)cf * Dims<DIM>::REC4 * 4, nrec * RB, bar);
-    }
+    mbar_expect_tx(bar, b4 + (2 + (HX ? 1 : 0)) * DIM * br + RS::bytes(a, nrec));
+    if (nrec) rs->issue(a, cf, nrec, bar);
     bulk_g2s(st.cell, a.S0.cell + base, b4, bar);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
@@ -514,9 +582,9 @@ __device__ __forceinline__ void stage_chunk(const StepArgs& a, AdvStage<DIM, Rea
 // restaging a buffer waits on no memory.  One barrier per chunk: the reads of
 // a buffer end there, and a ticket written after it is read only after the
 // next chunk's barrier.
-template <int DIM, typename Real, int CH, typename F>
+template <int DIM, typename Real, int CH, typename RS, typename F>
 __device__ __forceinline__ void staged_loop(const StepArgs& a, AdvStage<DIM, Real, CH>* st, uint64_t* bar, F&& f,
-                                            AdvRecStage<DIM>* rs = nullptr)
+                                            RS* rs)
 {
     __shared__ uint32_t tk[2];
     const uint32_t n = (uint32_t)a.stats->n_slots;
@@ -535,7 +603,7 @@ __device__ __forceinline__ void staged_loop(const StepArgs& a, AdvStage<DIM, Rea
             ChunkTicket t{atomicAdd(&a.stats->adv_next, 1u), 1u, 0u};
             ticket_cells<CH>(a, n, t, recs);
             tk[b] = t.tk;
-            if (t.tk < nchunks) stage_chunk<DIM, Real, CH>(a, st[b], &bar[b], t, n, recs ? rs + b : nullptr);
+            if (t.tk < nchunks) stage_chunk<DIM, Real, CH, RS>(a, st[b], &bar[b], t, n, recs ? rs + b : nullptr);
         }
         hand.tk = atomicAdd(&a.stats->adv_next, 1u);
     }
@@ -565,7 +633,7 @@ __device__ __forceinline__ void staged_loop(const StepArgs& a, AdvStage<DIM, Rea
             tk[sidx] = hand.tk;
             if (hand.tk < nchunks) {
                 fence_proxy_async();
-                stage_chunk<DIM, Real, CH>(a, st[sidx], &bar[sidx], hand, n, recs ? rs + sidx : nullptr);
+                stage_chunk<DIM, Real, CH, RS>(a, st[sidx], &bar[sidx], hand, n, recs ? rs + sidx : nullptr);
             }
             hand.tk = after;
         }
@@ -587,15 +655,18 @@ template <int DIM>
 __device__ __forceinline__ void velocity64(const double* __restrict__ Vc, uint32_t c, const double* xi, double* u)
 {
     constexpr int NV = 1 << DIM, VS = Dims<DIM>::VS;
-    const double* p = Vc + (size_t)c * NV * VS;
+    const double2* p = reinterpret_cast<const double2*>(Vc + (size_t)c * NV * VS);
     double N[NV];
     shape64<DIM>(xi, N);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) u[d] = 0.0;
 #pragma unroll
-    for (int iv = 0; iv < NV; ++iv)
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) u[d] = u[d] + N[iv] * __ldg(p + iv * VS + d);
+    for (int iv = 0; iv < NV; ++iv) {
+        const double2 a = __ldg(p + iv * (VS / 2));
+        u[0] = u[0] + N[iv] * a.x;
+        u[1] = u[1] + N[iv] * a.y;
+        if constexpr (DIM == 3) u[DIM - 1] = u[DIM - 1] + N[iv] * __ldg(p + iv * (VS / 2) + 1).x;
+    }
 }
 
 // The transport velocity of a sub-step from xi in cell c (vertices X).
@@ -622,15 +693,16 @@ __device__ __forceinline__ void transport64(const StepArgs& a, const double (*X)
 }
 
 // Sub-steps s0.. of one FP64 particle starting in cell c; returns the
-// sub-step at which it leaves its cell (S if it never does).
-template <int DIM, bool RK>
+// sub-step at which it leaves its cell (S if it never does).  LIN: the mesh's
+// cells are safe for locate_lin64.
+template <int DIM, bool RK, bool LIN = false>
 __device__ __forceinline__ int substeps64(const StepArgs& a, uint32_t c, int s0, double* x, double* xi, double* u,
                                           AdvCounters& k)
 {
     constexpr int NV = 1 << DIM;
     const MeshDev& m = a.mesh;
     double X[NV][DIM];
-    load_cell64<DIM>(m.cellX, c, X);
+    if constexpr (!LIN || RK) load_cell64<DIM>(m.cellX, c, X);
     int s = s0;
     for (; s < a.pp.S; ++s) {
         transport64<DIM, RK>(a, X, c, xi, u);
@@ -640,7 +712,10 @@ __device__ __forceinline__ int substeps64(const StepArgs& a, uint32_t c, int s0,
             x[d] = x[d] + st;
         }
         double xin[DIM];
-        const int st = inverse_map64<DIM>(X, m.aff + (size_t)c * Dims<DIM>::AFF, x, xin);
+        int st;
+        const double* ca = m.aff + (size_t)c * Dims<DIM>::AFF;
+        if constexpr (LIN) st = inverse_lin64<DIM>(m, [=](int j) { return __ldg(ca + j); }, c, x, xin);
+        else st = inverse_map64<DIM>(X, ca, x, xin);
         if (st) k.map_failures++;
         if (st == 0 && inside_unit<DIM>(xin)) {
 #pragma unroll
@@ -653,23 +728,53 @@ __device__ __forceinline__ int substeps64(const StepArgs& a, uint32_t c, int s0,
     return s;
 }
 
-constexpr int ADV64_CH = 512;
+constexpr uint32_t OWN_CELL = 0x80000000u;  // queued sub-step: the own cell's inverse map is still to be taken
 
-template <int DIM, bool RK>
-__global__ void __launch_bounds__(256) k_advect64(StepArgs a)
+constexpr int ADV64_CH = ADV_CH;  // the chunks whose first cells the seed and write passes record
+
+// Two doubles from shared memory, read where written: the compiler would
+// otherwise keep a cell's 24 velocities in registers over the sub-steps and
+// spill (702 us against 344 for the duct's 7.0 M particles: with 107 KB of
+// shared memory per block, spilled registers miss the small L1 that is left).
+__device__ __forceinline__ double2 lds2(const double* p)
+{
+    double2 t;
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(t.x), "=d"(t.y) : "r"(smem_u32(p)));
+    return t;
+}
+
+// velocity64 from a staged row of vertex velocities (4 doubles a vertex).
+__device__ __forceinline__ void velocity64_s(const double* V, const double* xi, double* u)
+{
+    double N[8];
+    shape64<3>(xi, N);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) u[d] = 0.0;
+#pragma unroll
+    for (int iv = 0; iv < 8; ++iv) {
+        const double2 t = lds2(V + 4 * iv), z = lds2(V + 4 * iv + 2);
+        u[0] = u[0] + N[iv] * t.x;
+        u[1] = u[1] + N[iv] * t.y;
+        u[2] = u[2] + N[iv] * z.x;
+    }
+}
+
+template <int DIM, bool RK, bool LIN>
+__global__ void __launch_bounds__(256, LIN ? 2 : 1) k_advect64(const __grid_constant__ StepArgs a)
 {
     pdl_entry();
     extern __shared__ __align__(128) unsigned char adv_raw[];
     __shared__ uint64_t bar[2];
     auto* st = reinterpret_cast<AdvStage<DIM, double, ADV64_CH>*>(adv_raw);
+    auto* rs = reinterpret_cast<AdvLin64Stage*>(adv_raw + 2 * sizeof(AdvStage<DIM, double, ADV64_CH>));
     const MeshDev& m = a.mesh;
     AdvCounters k;
-    staged_loop<DIM, double, ADV64_CH>(a, st, bar, [&](AdvStage<DIM, double, ADV64_CH>& sg, int, uint32_t t,
-                                                       uint32_t i, bool in) {
+    staged_loop<DIM, double, ADV64_CH, AdvLin64Stage>(a, st, bar, [&](AdvStage<DIM, double, ADV64_CH>& sg, int sidx,
+                                                                      uint32_t t, uint32_t i, bool in) {
         const uint32_t c = in ? sg.cell[t] : HOLE;
         const bool act = c != HOLE && in;
         bool want = false, counted = false;
-        int s = 0, pe = 0;
+        int s = 0, pe = 0, where = 0;
         if (in && c == HOLE) a.key[i] = LOST;
         if (act) {
             double x[DIM], xi[DIM], v[DIM], u[DIM];
@@ -682,13 +787,57 @@ __global__ void __launch_bounds__(256) k_advect64(StepArgs a)
             const bool alive = c < (uint32_t)m.nC;
             if (!alive) k.err |= ERR_BAD_CELL;
             if (alive) {
-                if (a.do_correct) {  // :126-138, deltaV = V - Vold per vertex
-                    double corr[DIM];
-                    velocity64<DIM>((const double*)a.dVc, c, xi, corr);
+                if constexpr (LIN) {
+                    const AdvLin64Stage& rsg = rs[sidx];
+                    const uint32_t lc = c - rsg.cfirst;
+                    const bool srec = a.chunk_first && lc < rsg.ncell;
+                    // V (or V - Vold) at y, from the stage or, where a chunk spans too many cells, from global memory
+                    auto field = [&](const double (*row)[AdvLin64Stage::VW], const void* all, const double* y, double* f) {
+                        if (srec) velocity64_s(row[lc], y, f);
+                        else velocity64<3>((const double*)all, c, y, f);
+                    };
+                    if (a.do_correct) {  // :126-138, deltaV = V - Vold per vertex
+                        field(rsg.dv, a.dVc, xi, u);
 #pragma unroll
-                    for (int d = 0; d < DIM; ++d) v[d] = v[d] + corr[d];
+                        for (int d = 0; d < 3; ++d) v[d] = v[d] + u[d];
+                    }
+                    for (; s < a.pp.S; ++s) {  // substeps64's operations
+                        field(rsg.v, a.Vc, xi, u);
+                        if constexpr (RK) {  // transport64's operations
+                            double X[8][3], J[3][3], Ji[3][3], dl[3], xm[3];
+                            load_cell64<3>(m.cellX, c, X);
+                            jac64<3>(X, xi, J);
+                            if (invert64<3>(J, Ji) > 0.0) {
+                                matvec64<3>(Ji, u, dl);
+                                const double half = a.pp.dtp * 0.5;
+#pragma unroll
+                                for (int d = 0; d < 3; ++d) xm[d] = xi[d] + half * dl[d];
+                                field(rsg.v, a.Vc, xm, u);
+                            }
+                        }
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) {
+                            const double sd = u[d] * a.pp.dtp;
+                            x[d] = x[d] + sd;
+                        }
+                        double xin[3];
+                        const double* ca = m.aff + (size_t)c * 12;
+                        where = srec ? locate_lin64([&](int j) { return rsg.aff[lc][j]; }, x, xin)
+                                     : locate_lin64([&](int j) { return __ldg(ca + j); }, x, xin);
+                        if (where) break;
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) xi[d] = xin[d];
+                        if (near_face_fast64(xin)) k.near_face++;
+                    }
+                } else {
+                    if (a.do_correct) {
+                        double corr[DIM];
+                        velocity64<DIM>((const double*)a.dVc, c, xi, corr);
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) v[d] = v[d] + corr[d];
+                    }
+                    s = substeps64<DIM, RK>(a, c, 0, x, xi, u, k);
                 }
-                s = substeps64<DIM, RK>(a, c, 0, x, xi, u, k);
                 want = s < a.pp.S;
             }
 #pragma unroll
@@ -705,16 +854,19 @@ __global__ void __launch_bounds__(256) k_advect64(StepArgs a)
                 if (counted) pe = ext_part<DIM, double>(xi, a.pp);
             }
         }
-        defer(a, want, i, s);
+        // a point that locate_lin64 leaves undecided is mapped by k_search64: the function calls of
+        // inverse_map64 here would spill the loop's registers (684 against 344 us
+        // for the duct's 7.0 M particles)
+        defer(a, want, i, where == 2 ? s | (int)OWN_CELL : s);
         count_cells(a, counted, c, pe);
-    });
+    }, LIN && a.chunk_first ? rs : nullptr);
     flush_counters(a, k);
 }
 
 // Deferred FP64 particles: the search of sub-step s (:438-491), then the
 // remaining sub-steps (searching again whenever needed).
-template <int DIM, bool RK>
-__global__ void __launch_bounds__(128) k_search64(StepArgs a)
+template <int DIM, bool RK, bool LIN>
+__global__ void __launch_bounds__(128) k_search64(const __grid_constant__ StepArgs a)
 {
     pdl_entry();
     const uint32_t nq = *a.nxq < a.capacity ? *a.nxq : a.capacity;
@@ -723,7 +875,7 @@ __global__ void __launch_bounds__(128) k_search64(StepArgs a)
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
         const uint2 e = a.xq[q];
         const uint32_t i = e.x;
-        int s = (int)e.y;
+        int s = (int)(e.y & ~OWN_CELL);
         uint32_t c = a.key[i];
         const uint32_t c_old = a.S0.cell[i];
         double x[DIM], xi[DIM], u[DIM];
@@ -733,7 +885,25 @@ __global__ void __launch_bounds__(128) k_search64(StepArgs a)
             xi[d] = ((const double*)a.T.xi[d])[i];
         }
         bool alive = true;
-        while (true) {
+        if constexpr (LIN) {
+            if (e.y & OWN_CELL) {
+                double xin[DIM];
+                Vec<DIM> p;
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) p.v[d] = x[d];
+                const InvOut<DIM> o = inverse_full64<DIM>(m.cellX, m.aff, c, p);
+                if (o.st) k.map_failures++;
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) xin[d] = o.xi[d];
+                if (o.st == 0 && inside_unit<DIM>(xin)) {
+                    if (near_face64<DIM>(xin)) k.near_face++;
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) xi[d] = xin[d];
+                    s = substeps64<DIM, RK, LIN>(a, c, s + 1, x, xi, u, k);
+                }
+            }
+        }
+        while (s < a.pp.S) {
             // velocity_ext of sub-step s, recomputed from the start-of-sub-step state
             if constexpr (RK) {
                 double X[1 << DIM][DIM];
@@ -749,7 +919,7 @@ __global__ void __launch_bounds__(128) k_search64(StepArgs a)
                 ve.v[d] = u[d];
                 xp.v[d] = x[d];
             }
-            const SearchOut so = search64<DIM>(m, c, xo, ve, xp);
+            const SearchOut so = search64<DIM, false, LIN>(m, c, xo, ve, xp);
             k.searched++;
             k.map_failures += so.map_failures;
             if (so.flags & SRCH_OVERFLOW) k.err |= ERR_CAND_OVERFLOW;
@@ -761,8 +931,7 @@ __global__ void __launch_bounds__(128) k_search64(StepArgs a)
             c = so.cell;
 #pragma unroll
             for (int d = 0; d < DIM; ++d) xi[d] = so.xi[d];
-            s = substeps64<DIM, RK>(a, c, s + 1, x, xi, u, k);
-            if (s >= a.pp.S) break;
+            s = substeps64<DIM, RK, LIN>(a, c, s + 1, x, xi, u, k);
         }
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
@@ -918,7 +1087,7 @@ struct SubOut {
 };
 
 template <int DIM>
-__device__ __noinline__ SubOut<DIM> twisted_substeps32(const float* __restrict__ geo, uint32_t c, int s0, int S,
+__device__ __forceinline__ SubOut<DIM> twisted_substeps32(const float* __restrict__ geo, uint32_t c, int s0, int S,
                                                        float dtp, const Rec32<DIM> r, F3<DIM> x0)
 {
     Geo32<DIM> g;

@@ -29,8 +29,8 @@ struct pfem2gpu_handle {
             *d2c_ent = nullptr;
     double *verts = nullptr, *cellX = nullptr, *aff = nullptr, *v2c_dirs = nullptr;
     float* geo32 = nullptr;
-    uint32_t* twisted = nullptr;  // cells whose map is not affine (set by cell_setup)
-    bool all_affine = false;
+    uint32_t* twisted = nullptr;  // cells whose map is not affine; 3D cells unfit for locate_lin64 (set by cell_setup)
+    bool all_affine = false, lin64 = false;
     // velocities
     double *Vstage = nullptr, *Vstage2 = nullptr, *Vout = nullptr;
     double* Vin = nullptr;  // host V of the current call, uploaded before its check (see stage_v)
@@ -49,7 +49,7 @@ struct pfem2gpu_handle {
     uint32_t *carr = nullptr, *carrs = nullptr, *ccount = nullptr;
     unsigned long long *cocc = nullptr, *cub = nullptr, *coff = nullptr, *tiles64 = nullptr;
     uint4* gscr = nullptr;
-    uint32_t* chunk_first = nullptr;  // FP32 form: first cell of each advect chunk of the current layout
+    uint32_t* chunk_first = nullptr;  // first cell of each advect chunk of the current layout
     float *jinv32 = nullptr, *vrec32 = nullptr, *dvrec32 = nullptr;
     bool launch_failed = false;
     // CUDA graphs of the per-step sequences (one per buffer parity and
@@ -214,6 +214,7 @@ StepArgs args(pfem2gpu_handle* h)
     StepArgs a{};
     a.mesh.nC = h->nC;
     a.mesh.all_affine = h->all_affine ? 1 : 0;
+    a.mesh.lin64 = h->lin64 ? 1 : 0;
     a.mesh.nV = h->nV;
     a.mesh.nD = h->nD;
     a.mesh.cv = h->cv;
@@ -378,12 +379,10 @@ int ensure_capacity(pfem2gpu_handle* h, uint64_t need, uint64_t want = 0)
     CK(alloc_state(h, nt, (uint32_t)cap, false));
     uint32_t* cf_new = nullptr;
     const size_t ncf = (cap + ADV_CH - 1) / ADV_CH + 1;
-    if (h->prec == PFEM2GPU_FP32) {
-        CK(dalloc(&cf_new, ncf));
-        if (h->chunk_first)
-            CK(cudaMemcpyAsync(cf_new, h->chunk_first, ((size_t)h->cap + ADV_CH - 1) / ADV_CH * 4 + 4,
-                               cudaMemcpyDeviceToDevice, h->stream));
-    }
+    CK(dalloc(&cf_new, ncf));
+    if (h->chunk_first)
+        CK(cudaMemcpyAsync(cf_new, h->chunk_first, ((size_t)h->cap + ADV_CH - 1) / ADV_CH * 4 + 4,
+                           cudaMemcpyDeviceToDevice, h->stream));
     if (h->S0.cell && h->has_particles) {
         const size_t n = h->cap, es = esize(h);
         CK(cudaMemcpyAsync(n0.cell, h->S0.cell, n * 4, cudaMemcpyDeviceToDevice, h->stream));
@@ -1155,8 +1154,8 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
         CK(cudaMemsetAsync(h->dvrec32, 0, nc * rec * 4, h->stream));
     }
     CK(dalloc(&h->jinv32, nc * (dim == 3 ? 12 : 8)));
-    CK(dalloc(&h->twisted, 1));
-    CK(cudaMemsetAsync(h->twisted, 0, 4, h->stream));
+    CK(dalloc(&h->twisted, 2));
+    CK(cudaMemsetAsync(h->twisted, 0, 8, h->stream));
     CK(cudaMalloc(&h->partials, nc * PW * esize(h)));
     CK(cudaMemcpyAsync(h->cv, cell_vertices, nc * NV * 4, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->cd, cell_dofs, nc * NV * 4, cudaMemcpyHostToDevice, h->stream));
@@ -1171,10 +1170,11 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
             return launch_cell_setup(dim, h->nC, h->verts, h->cv, h->cellX, h->aff, h->geo32, h->jinv32, h->twisted,
                                      h->stream);
         });
-    uint32_t twisted = 0;
-    CK(cudaMemcpyAsync(&twisted, h->twisted, 4, cudaMemcpyDeviceToHost, h->stream));
+    uint32_t twisted[2] = {0, 0};
+    CK(cudaMemcpyAsync(twisted, h->twisted, 8, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));  // host vectors above go out of scope
-    h->all_affine = twisted == 0;
+    h->all_affine = twisted[0] == 0;
+    h->lin64 = dim == 3 && twisted[1] == 0;
     h->has_mesh = true;
     h->vaos_valid = false;
     h->gen++;

@@ -22,7 +22,7 @@ constexpr int NPE_MAX = 256;   // extended cell parts (q0+1)(q1+1)(q2+1)
 constexpr int OCCW_MAX = 4;    // 64-bit part-occupancy words per cell
 constexpr int ARRCAP = 32;     // arrival slots per cell before the overflow list
 constexpr int CELL_WARPS = 4;  // warps per block of the warp-per-cell helper kernels
-constexpr int ADV_CH = 512;    // particles per staged chunk of the FP32 advect pass
+constexpr int ADV_CH = 512;    // particles per staged chunk of the advect pass
 // cells whose velocity records an FP32 advect chunk stages with its particles
 // (a chunk spans about ADV_CH / particles-per-cell + 1 cells; beyond this
 // many, the chunk's particles read their records from global memory)
@@ -62,6 +62,7 @@ struct DevStats {
 struct MeshDev {
     int nC, nV, nD;
     int all_affine;           // 1 if every cell's multilinear map is affine (no twist terms)
+    int lin64;                // 3D: 1 if locate_lin64 holds for every cell
     const int32_t* cv;        // nC x NV vertex ids
     const int32_t* cd;        // nC x NV DoF ids
     const double* cellX;      // nC x NV x DIM vertex coordinates, cell-major

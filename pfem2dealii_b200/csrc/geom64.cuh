@@ -164,6 +164,24 @@ __device__ __forceinline__ bool near_face64(const double* xi)
     return nf;
 }
 
+// The same two tests (3D), most points decided by integer compares of the
+// high words: below that of 1.0 a double is in [0, 1), between those of
+// 1e-12 and the last one below 1.0 it is near neither face.
+__device__ __forceinline__ bool inside_fast64(const double* xi)
+{
+    const bool sure = (unsigned)__double2hiint(xi[0]) < 0x3FF00000u && (unsigned)__double2hiint(xi[1]) < 0x3FF00000u &&
+                      (unsigned)__double2hiint(xi[2]) < 0x3FF00000u;
+    return sure || inside_unit<3>(xi);
+}
+__device__ __forceinline__ bool near_face_fast64(const double* xi)
+{
+    bool maybe = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        maybe = maybe || (unsigned)__double2hiint(xi[d]) - 0x3D71979Au >= 0x3FEFFFFFu - 0x3D71979Au;
+    return maybe && near_face64<3>(xi);
+}
+
 // 2D closed-form bilinear inverse: r = xi e + eta f + xi eta g with
 // e = X1-X0, f = X2-X0, g = X3-X1-X2+X0, r = p-X0; eliminating xi leaves
 // cross(f,g) eta^2 + (cross(f,e) - cross(r,g)) eta - cross(r,e) = 0, solved
@@ -351,6 +369,72 @@ __device__ __forceinline__ int inverse_affine64(const double* __restrict__ aff, 
         xi[k] = acc;
     }
     return 0;
+}
+
+// Decides inverse_map64 of a hex from its affine guess g = A^-1 (p - b) alone
+// (the same operations in the same order): 0, inside, with xi = g, the value
+// inverse_map64 returns; 1, outside, where it returns a point outside the
+// unit cell; 2, undecided.  Only for cells that cell_setup found safe (LIN64_MAX):
+// the map is affine and all its roundings together move a point by less than
+// 1e-11 / sqrt(3) in reference coordinates for points up to half a cell outside,
+// so that a guess inside the cell needs no clamping and its weighted residual
+// passes Newton's first test (|J^-1 f|^2 <= 1e-22), and a guess more than 1e-9
+// outside leads, after clamping, to one Newton step that lands within 1e-11
+// of it and stops.  What is left out is the residual F(g) - p, the Jacobian
+// and its inverse: 250 of the 340 FP64 operations of a sub-step.
+constexpr double LIN64_MAX = 3e-12;
+template <typename Aff>  // aff(j): the cell's j-th affine value
+__device__ __forceinline__ int locate_lin64(Aff&& aff, const double* p, double* xi)
+{
+    double r[3], g[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) r[d] = p[d] - aff(9 + d);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        double acc = 0.0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) acc = acc + aff(k * 3 + d) * r[d];
+        g[k] = acc;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) xi[d] = g[d];
+    if (inside_fast64(g)) return 0;
+    bool out = false, near = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        out = out || g[d] < -1e-9 || g[d] > 1.0 + 1e-9;
+        near = near && (g[d] >= -0.5 && g[d] <= 1.5);
+    }
+    return out && near ? 1 : 2;
+}
+
+// The largest reference-coordinate error of one hex's maps where it is affine
+// (the bound of locate_lin64), infinity where it is not: rounding of the
+// forward map up to half a cell outside (11 roundings of sum |N| |X| <= 8 xm)
+// and of b (12), times |A^-1|, and the inverses' own (about cond^2 roundings).
+__device__ __forceinline__ double lin64_error(const double (*X)[3], const double* aff, bool affine)
+{
+    constexpr double u = 1.1102230246251565e-16;
+    double xm = 0.0, na = 0.0, nA = 0.0;
+    for (int i = 0; i < 8; ++i)
+        for (int d = 0; d < 3; ++d) xm = fmax(xm, fabs(X[i][d]));
+    for (int k = 0; k < 3; ++k) {
+        double s = 0.0, t = 0.0;
+        for (int d = 0; d < 3; ++d) {
+            s += fabs(aff[k * 3 + d]);
+            t += fabs(X[1][k] - X[0][k]) * (d == 0) + fabs(X[2][k] - X[0][k]) * (d == 1) + fabs(X[4][k] - X[0][k]) * (d == 2);
+        }
+        na = fmax(na, s);
+        nA = fmax(nA, t);
+    }
+    // det A > 0, as Newton asks of the Jacobian
+    double e[3][3];
+    for (int d = 0; d < 3; ++d)
+        for (int k = 0; k < 3; ++k) e[d][k] = X[1 << k][d] - X[0][d];
+    const double det = e[0][0] * (e[1][1] * e[2][2] - e[1][2] * e[2][1]) - e[0][1] * (e[1][0] * e[2][2] - e[1][2] * e[2][0]) +
+                       e[0][2] * (e[1][0] * e[2][1] - e[1][1] * e[2][0]);
+    const double cond = na * nA, err = na * 100.0 * u * xm + 40.0 * u * cond * cond;
+    return affine && det > 0.0 && err == err ? err : __longlong_as_double(0x7ff0000000000000ll);
 }
 
 template <int DIM>

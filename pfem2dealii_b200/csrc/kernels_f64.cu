@@ -76,6 +76,8 @@ __global__ void k_cell_setup(int nC, const double* __restrict__ verts, const int
         for (int k = DIM * DIM; k < JS; ++k) jj[k] = 0.0f;
         jj[DIM * DIM] = affine ? 1.0f : 0.0f;
         if (!affine) atomicAdd(twisted, 1u);
+        if constexpr (DIM == 3)
+            if (!(lin64_error(X, aff + (size_t)c * Dims<DIM>::AFF, affine) <= LIN64_MAX)) atomicAdd(twisted + 1, 1u);
     }
 }
 
@@ -120,18 +122,29 @@ static int smem_grid(K kernel, int threads, int smem)
 
 // RK: the midpoint sub-step (params.integrator = PFEM2GPU_RK2), compiled as
 // its own kernels so that the Euler ones carry no trace of it.
+template <int DIM, bool RK, bool LIN>
+static int advect_l(const StepArgs& a, cudaStream_t s)
+{
+    const int smem = 2 * (int)(sizeof(AdvStage<DIM, double, ADV64_CH>) + (LIN ? sizeof(AdvLin64Stage) : 0));
+    static const int grid = smem_grid(k_advect64<DIM, RK, LIN>, 256, smem);
+    return launch_pdl(k_advect64<DIM, RK, LIN>, grid, 256, smem, s, a);
+}
+
 template <int DIM, bool RK>
 static int advect_t(const StepArgs& a, cudaStream_t s)
 {
-    const int smem = 2 * (int)sizeof(AdvStage<DIM, double, ADV64_CH>);
-    static const int grid = smem_grid(k_advect64<DIM, RK>, 256, smem);
-    return launch_pdl(k_advect64<DIM, RK>, grid, 256, smem, s, a);
+    if constexpr (DIM == 3)
+        if (a.mesh.lin64) return advect_l<DIM, RK, true>(a, s);
+    return advect_l<DIM, RK, false>(a, s);
 }
 
 template <int DIM, bool RK>
 static int search_t(const StepArgs& a, cudaStream_t s)
 {
-    return launch_pdl(k_search64<DIM, RK>, PFEM2_GRID((k_search64<DIM, RK>), 128), 128, 0, s, a);
+    if constexpr (DIM == 3)
+        if (a.mesh.lin64)
+            return launch_pdl(k_search64<DIM, RK, true>, PFEM2_GRID((k_search64<DIM, RK, true>), 128), 128, 0, s, a);
+    return launch_pdl(k_search64<DIM, RK, false>, PFEM2_GRID((k_search64<DIM, RK, false>), 128), 128, 0, s, a);
 }
 
 int launch64_advect(int dim, const StepArgs& a, cudaStream_t s)
