@@ -27,12 +27,13 @@ struct pfem2gpu_handle {
     bool has_mesh = false;
     int32_t *cv = nullptr, *cd = nullptr, *v2c_off = nullptr, *v2c_cells = nullptr, *d2c_off = nullptr,
             *d2c_ent = nullptr;
-    double *verts = nullptr, *cellX = nullptr, *aff = nullptr, *v2c_dirs = nullptr;
+    double *verts = nullptr, *cellX = nullptr, *aff = nullptr, *v2c_dirs = nullptr, *v2c_rec = nullptr;
     float* geo32 = nullptr;
     uint32_t* twisted = nullptr;  // cells whose map is not affine; 3D cells unfit for locate_lin64 (set by cell_setup)
     bool all_affine = false, lin64 = false;
     // velocities
     double *Vstage = nullptr, *Vstage2 = nullptr, *Vout = nullptr;
+    double* Va = nullptr;  // the staged V, one row per DoF
     double* Vin = nullptr;  // host V of the current call, uploaded before its check (see stage_v)
     unsigned* nf_h = nullptr;  // mapped host word: the uploaded V holds a non-finite value
     unsigned* nf_d = nullptr;  // its device address
@@ -224,8 +225,7 @@ StepArgs args(pfem2gpu_handle* h)
     a.mesh.geo32 = h->geo32;
     a.mesh.jinv32 = h->jinv32;
     a.mesh.v2c_off = h->v2c_off;
-    a.mesh.v2c_cells = h->v2c_cells;
-    a.mesh.v2c_dirs = h->v2c_dirs;
+    a.mesh.v2c_rec = h->v2c_rec;
     a.mesh.d2c_off = h->d2c_off;
     a.mesh.d2c_ent = h->d2c_ent;
     a.pp = h->pp;
@@ -236,7 +236,7 @@ StepArgs args(pfem2gpu_handle* h)
     a.dVc = h->dVc;
     a.vrec32 = h->vrec32;
     a.dvrec32 = h->dvrec32;
-    a.Vd = h->Vstage;
+    a.Va = h->Va;
     a.do_correct = 0;
     a.apply_counts = 1;
     a.key = h->key;
@@ -474,12 +474,12 @@ int stage_v(pfem2gpu_handle* h, const double* V, const double* Vold, bool device
     if (h->prec == PFEM2GPU_FP64) {
         run(h, "stage_velocity", [&] {
             return launch_cell_v(h->dim, h->prec, v, vo, h->cd, h->nC, h->nD, h->Vc, Vold ? h->dVc : nullptr, vcopy,
-                                 h->stream);
+                                 h->Va, h->stream);
         });
     } else {
         run(h, "stage_velocity", [&] {
             return launch_cell_rec32(h->dim, v, vo, h->cd, h->aff, h->jinv32, h->nC, h->nD, h->vrec32,
-                                     Vold ? h->dvrec32 : nullptr, vcopy, h->stream);
+                                     Vold ? h->dvrec32 : nullptr, vcopy, h->Va, h->stream);
         });
     }
     h->vaos_valid = true;
@@ -790,7 +790,7 @@ int window_forward_impl(pfem2gpu_handle* h, int K, int C, const double* V, const
     WinArgs w = winargs(h);
     run(h, "window_cells", [&] {
         return launch_cell_v(h->dim, 0, W.V, Vold ? W.Vold : nullptr, h->cd, h->nC, h->nD, W.Vcell, W.dVcell,
-                             nullptr, h->stream) +
+                             nullptr, nullptr, h->stream) +
                launch_win_wcell(h->dim, w, W.Vcell, W.Wcell, h->stream);
     });
     run(h, "window_compact", [&] { return launch_win_compact(h->S0.cell, ns, (uint32_t)h->nC, W.tsum, W.slot, h->stream); });
@@ -974,7 +974,7 @@ int pfem2gpu_destroy(pfem2gpu_handle* h)
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (void* p : {(void*)h->cv, (void*)h->cd, (void*)h->v2c_off, (void*)h->v2c_cells, (void*)h->d2c_off,
                     (void*)h->d2c_ent, (void*)h->verts, (void*)h->cellX, (void*)h->aff, (void*)h->v2c_dirs,
-                    (void*)h->geo32, (void*)h->Vstage, (void*)h->Vstage2, (void*)h->Vout, (void*)h->Vin, h->Vc, h->dVc,
+                    (void*)h->geo32, (void*)h->v2c_rec, (void*)h->Va, (void*)h->Vstage, (void*)h->Vstage2, (void*)h->Vout, (void*)h->Vin, h->Vc, h->dVc,
                     (void*)h->key, (void*)h->next, (void*)h->xtmp, (void*)h->head, (void*)h->cs0, (void*)h->cs1,
                     (void*)h->carr, (void*)h->carrs, (void*)h->ccount, (void*)h->cocc, (void*)h->cub, (void*)h->coff,
                     (void*)h->tiles64, (void*)h->gscr, (void*)h->jinv32, (void*)h->xq, (void*)h->nxq,
@@ -1050,6 +1050,9 @@ static cudaError_t build_maps(pfem2gpu_handle* h, size_t nc, size_t nvx, size_t 
         BM(cudaMemcpyAsync(h->v2c_off, v2c_offsets, (nvx + 1) * 4, cudaMemcpyHostToDevice, s));
         BM(cudaMemcpyAsync(h->v2c_cells, v2c_cells, (size_t)total * 4, cudaMemcpyHostToDevice, s));
         BM(cudaMemcpyAsync(h->v2c_dirs, v2c_dirs, (size_t)total * dim * 8, cudaMemcpyHostToDevice, s));
+        BM(dalloc(&h->v2c_rec, std::max<size_t>((size_t)total * 4, 4)));
+        launch_v2c_pack(dim, (size_t)total, h->v2c_cells, h->v2c_dirs, h->v2c_rec, s);
+        BM(cudaGetLastError());
         BM(cudaStreamSynchronize(s));
         return done(cudaSuccess);
     }
@@ -1064,6 +1067,8 @@ static cudaError_t build_maps(pfem2gpu_handle* h, size_t nc, size_t nvx, size_t 
     BM(dalloc(&h->v2c_dirs, std::max<size_t>((size_t)total * dim, 1)));
     launch_v2c_build(dim, (int)nc, (int)nvx, h->verts, h->cv, (const uint32_t*)h->v2c_off, fill, h->v2c_cells,
                      h->v2c_dirs, s);
+    BM(dalloc(&h->v2c_rec, std::max<size_t>((size_t)total * 4, 4)));
+    launch_v2c_pack(dim, (size_t)total, h->v2c_cells, h->v2c_dirs, h->v2c_rec, s);
     BM(cudaGetLastError());
     BM(cudaStreamSynchronize(s));
 #undef BM
@@ -1099,7 +1104,8 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
     // release an older mesh (a failure further down leaves no dangling pointer)
     for (void** p : {(void**)&h->cv, (void**)&h->cd, (void**)&h->v2c_off, (void**)&h->v2c_cells, (void**)&h->d2c_off,
                      (void**)&h->d2c_ent, (void**)&h->verts, (void**)&h->cellX, (void**)&h->aff,
-                     (void**)&h->v2c_dirs, (void**)&h->geo32, (void**)&h->Vstage, (void**)&h->Vstage2,
+                     (void**)&h->v2c_dirs, (void**)&h->v2c_rec, (void**)&h->Va, (void**)&h->geo32, (void**)&h->Vstage,
+                     (void**)&h->Vstage2,
                      (void**)&h->Vout, (void**)&h->Vin, (void**)&h->Vc, (void**)&h->dVc, (void**)&h->head, (void**)&h->cs0,
                      (void**)&h->cs1, (void**)&h->carr, (void**)&h->carrs, (void**)&h->ccount, (void**)&h->cocc,
                      (void**)&h->cub, (void**)&h->coff, (void**)&h->tiles64, (void**)&h->jinv32, (void**)&h->vrec32,
@@ -1126,6 +1132,7 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
     CK(dalloc(&h->aff, nc * AFF));
     CK(dalloc(&h->geo32, nc * GS));
     CK(dalloc(&h->Vstage, nd * dim));
+    CK(dalloc(&h->Va, nd * VS));
     CK(dalloc(&h->Vstage2, nd * dim));
     CK(dalloc(&h->Vin, nd * dim));
     CK(dalloc(&h->Vout, nd * dim));
@@ -1165,6 +1172,7 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
     CK(cudaMemsetAsync(h->dVc, 0, vcn * esize(h), h->stream));
     run(h, "fill", [&] { return launch_fill_u32(h->head, (uint32_t)nc, LOST, h->stream); });
     CK(cudaMemsetAsync(h->Vstage, 0, nd * dim * 8, h->stream));
+    CK(cudaMemsetAsync(h->Va, 0, nd * VS * 8, h->stream));
     run(h, "cell_setup",
         [&] {
             return launch_cell_setup(dim, h->nC, h->verts, h->cv, h->cellX, h->aff, h->geo32, h->jinv32, h->twisted,

@@ -70,7 +70,7 @@ __device__ __forceinline__ void new_particle_at(const StepArgs& a, uint32_t c, c
         xid[d] = (idx[d] + 0.5) * a.pp.h[d];
         xi[d] = (Real)xid[d];
     }
-    velocity_from_dofs<DIM>(a.mesh.cd, a.Vd, a.mesh.nD, c, xid, vd);
+    velocity_from_dofs<DIM>(a.mesh.cd, a.Va, c, xid, vd);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) v[d] = (Real)vd[d];
     if constexpr (std::is_same<Real, double>::value) {

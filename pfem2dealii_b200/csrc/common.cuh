@@ -70,8 +70,7 @@ struct MeshDev {
     const float* geo32;       // nC x GEO: FP32 multilinear coefficients relative to vertex 0
     const float* jinv32;      // nC x JS: FP32 inverse Jacobian at the centre, then the affine flag
     const int32_t* v2c_off;   // nV + 1
-    const int32_t* v2c_cells; // cells around each vertex, ascending
-    const double* v2c_dirs;   // DIM per entry: unit vertex -> cell-centre direction
+    const double* v2c_rec;    // 4 doubles per entry: unit vertex -> cell-centre direction (DIM), then the cell's bits
     const int32_t* d2c_off;   // nD + 1
     const int32_t* d2c_ent;   // cell * NV + local vertex, cells ascending
 };
@@ -109,7 +108,7 @@ struct StepArgs {
     const void* dVc;    // FP64 form: nC x NV x VS velocity increment V - Vold per cell vertex
     const float* vrec32;  // FP32 form: nC x REC4 float4, velocity polynomial of each cell (+ affine flag)
     const float* dvrec32; // FP32 form: nC x REC4 float4, polynomial of V - Vold
-    const double* Vd;     // staged nodal velocity, component-major (nD per component)
+    const double* Va;     // staged nodal velocity, nD x VS (one row per DoF)
     int do_correct;
     int apply_counts;   // write kernel: 1 = count correction, 0 = keep all (re-sort only)
     int count_step;     // write kernel: add the step's particles to particle_steps
@@ -145,7 +144,7 @@ constexpr int WIN_TILE = 1024;          // elements per tile of the window scans
 constexpr uint32_t ERR_REPLAY = 128u;   // backward: a recomputed segment ended elsewhere than its checkpoint
 
 struct WinArgs {
-    StepArgs a;                // mesh, parameters, staged velocities (Vc/dVc or vrec32/dvrec32, Vd = V)
+    StepArgs a;                // mesh, parameters, staged velocities (Vc/dVc or vrec32/dvrec32, Va = V)
     uint32_t n;                // particles in the window
     int K, C, nseg;            // steps, steps per segment, segments
     int do_correct;            // 1: correction with V - Vold every step

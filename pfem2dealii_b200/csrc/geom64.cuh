@@ -262,6 +262,34 @@ __device__ __forceinline__ void affine_setup64(const double (*X)[DIM], double* a
     for (int d = 0; d < DIM; ++d) aff[DIM * DIM + d] = b[d];
 }
 
+// A row of N doubles (N even, the row 16-byte aligned) in 16-byte loads: a
+// relocation's lanes read rows of different cells, and every load is a
+// request per lane whatever its width.
+template <int N>
+__device__ __forceinline__ void load_row64(const double* __restrict__ p, double* b)
+{
+#pragma unroll
+    for (int j = 0; j < N; j += 2) {
+        const double2 t = __ldg(reinterpret_cast<const double2*>(p + j));
+        b[j] = t.x;
+        b[j + 1] = t.y;
+    }
+}
+
+// The N ids (4 or 8) of one cell's row.
+template <int N>
+__device__ __forceinline__ void load_ids(const int32_t* __restrict__ p, int32_t* id)
+{
+#pragma unroll
+    for (int j = 0; j < N; j += 4) {
+        const int4 t = __ldg(reinterpret_cast<const int4*>(p + j));
+        id[j] = t.x;
+        id[j + 1] = t.y;
+        id[j + 2] = t.z;
+        id[j + 3] = t.w;
+    }
+}
+
 // MappingQ1::transform_real_to_unit_cell restated (deal.II's published
 // strategy): 2D closed form accepted inside the unit cell within 1e-12;
 // otherwise Newton from the affine guess clamped to the unit cell, residual
@@ -282,14 +310,15 @@ __device__ __forceinline__ int inverse_map64(const double (*X)[DIM], const doubl
         }
     }
     {
-        double Ai[DIM][DIM];
+        double Ai[DIM][DIM], row[DIM * DIM + DIM];
+        load_row64<DIM * DIM + DIM>(aff, row);
 #pragma unroll
         for (int k = 0; k < DIM; ++k)
 #pragma unroll
-            for (int d = 0; d < DIM; ++d) Ai[k][d] = aff[k * DIM + d];
+            for (int d = 0; d < DIM; ++d) Ai[k][d] = row[k * DIM + d];
         if (Ai[0][0] != Ai[0][0]) return 1;
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) r[d] = p[d] - aff[DIM * DIM + d];
+        for (int d = 0; d < DIM; ++d) r[d] = p[d] - row[DIM * DIM + d];
         matvec64<DIM>(Ai, r, xi);
     }
 #pragma unroll
@@ -356,16 +385,17 @@ __device__ __forceinline__ int inverse_map64(const double (*X)[DIM], const doubl
 template <int DIM>
 __device__ __forceinline__ int inverse_affine64(const double* __restrict__ aff, const double* p, double* xi)
 {
-    const double a00 = __ldg(aff);
-    if (a00 != a00) return 1;
+    double row[DIM * DIM + DIM];
+    load_row64<DIM * DIM + DIM>(aff, row);
+    if (row[0] != row[0]) return 1;
     double r[DIM];
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) r[d] = p[d] - __ldg(aff + DIM * DIM + d);
+    for (int d = 0; d < DIM; ++d) r[d] = p[d] - row[DIM * DIM + d];
 #pragma unroll
     for (int k = 0; k < DIM; ++k) {
         double acc = 0.0;
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) acc = acc + __ldg(aff + k * DIM + d) * r[d];
+        for (int d = 0; d < DIM; ++d) acc = acc + row[k * DIM + d] * r[d];
         xi[k] = acc;
     }
     return 0;
@@ -440,30 +470,35 @@ __device__ __forceinline__ double lin64_error(const double (*X)[3], const double
 template <int DIM>
 __device__ __forceinline__ void load_cell64(const double* __restrict__ cellX, uint32_t c, double (*X)[DIM])
 {
-    const double* p = cellX + (size_t)c * ((1 << DIM) * DIM);
+    constexpr int N = (1 << DIM) * DIM;  // 8 or 24 doubles: whole 16-byte pieces
+    double b[N];
+    load_row64<N>(cellX + (size_t)c * N, b);
 #pragma unroll
     for (int i = 0; i < (1 << DIM); ++i)
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) X[i][d] = __ldg(p + i * DIM + d);
+        for (int d = 0; d < DIM; ++d) X[i][d] = b[i * DIM + d];
 }
 
-// u = sum_i N_i(xi) V[d][dof_i] from the staged component-major nodal
-// vectors (V_d[dof] at Vd + d*nD), accumulated from zero in vertex order:
-// the reference's interpolation (src/pfem2particlehandler.cpp:96-101).
+// u = sum_i N_i(xi) V[dof_i] from the staged nodal velocities (VS doubles per
+// DoF), accumulated from zero in vertex order: the reference's interpolation
+// (src/pfem2particlehandler.cpp:96-101).
 template <int DIM>
-__device__ __forceinline__ void velocity_from_dofs(const int32_t* __restrict__ cd, const double* __restrict__ Vd,
-                                                   int nD, uint32_t c, const double* xi, double* u)
+__device__ __forceinline__ void velocity_from_dofs(const int32_t* __restrict__ cd, const double* __restrict__ Va,
+                                                   uint32_t c, const double* xi, double* u)
 {
-    constexpr int NV = 1 << DIM;
+    constexpr int NV = 1 << DIM, VS = Dims<DIM>::VS;
     double N[NV];
     shape64<DIM>(xi, N);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) u[d] = 0.0;
+    int32_t dof[NV];
+    load_ids<NV>(cd + (size_t)c * NV, dof);
 #pragma unroll
     for (int iv = 0; iv < NV; ++iv) {
-        const int32_t dof = __ldg(cd + (size_t)c * NV + iv);
+        double v[VS];
+        load_row64<VS>(Va + (size_t)dof[iv] * VS, v);
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) u[d] = u[d] + N[iv] * __ldg(Vd + (size_t)d * nD + dof);
+        for (int d = 0; d < DIM; ++d) u[d] = u[d] + N[iv] * v[d];
     }
 }
 

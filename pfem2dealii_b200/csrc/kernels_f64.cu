@@ -283,6 +283,18 @@ __global__ void k_v2c_finish(int nV, const double* __restrict__ verts, const int
     }
 }
 
+// Direction and cell of every entry in one 32-byte record.
+template <int DIM>
+__global__ void k_v2c_pack(size_t n, const int32_t* __restrict__ cells, const double* __restrict__ dirs,
+                           double* __restrict__ rec)
+{
+    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+            rec[4 * k + d] = d < DIM ? dirs[k * DIM + d] : d == DIM ? __hiloint2double(0, cells[k]) : 0.0;
+    }
+}
+
 // dof -> (cell, local vertex) entries k = cell * NV + i, ascending per dof.
 __global__ void k_d2c_count(long long nE, const int32_t* __restrict__ cd, uint32_t* __restrict__ cnt)
 {
@@ -352,6 +364,13 @@ int launch_v2c_build(int dim, int nC, int nV, const double* verts, const int32_t
         k_v2c_finish<3><<<PFEM2_GRID(k_v2c_finish<3>, 128), 128, 0, s>>>(nV, verts, cv, off, cells, dirs);
     }
     return 2;
+}
+
+int launch_v2c_pack(int dim, size_t n, const int32_t* cells, const double* dirs, double* rec, cudaStream_t s)
+{
+    if (dim == 2) k_v2c_pack<2><<<PFEM2_GRID(k_v2c_pack<2>, 256), 256, 0, s>>>(n, cells, dirs, rec);
+    else k_v2c_pack<3><<<PFEM2_GRID(k_v2c_pack<3>, 256), 256, 0, s>>>(n, cells, dirs, rec);
+    return 1;
 }
 
 static int grid_n64(size_t n, int threads)

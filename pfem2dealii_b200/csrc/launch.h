@@ -76,6 +76,7 @@ int launch_pack_output(int dim, int prec, const StepArgs& a, const uint32_t* slo
 int launch_v2c_count(int dim, int nC, const int32_t* cv, uint32_t* cnt, cudaStream_t s);
 int launch_v2c_build(int dim, int nC, int nV, const double* verts, const int32_t* cv, const uint32_t* off,
                      uint32_t* fill, int32_t* cells, double* dirs, cudaStream_t s);
+int launch_v2c_pack(int dim, size_t n, const int32_t* cells, const double* dirs, double* rec, cudaStream_t s);
 int launch_d2c_count(long long nE, const int32_t* cd, uint32_t* cnt, cudaStream_t s);
 int launch_d2c_build(long long nE, int nD, const int32_t* cd, const uint32_t* off, uint32_t* fill, int32_t* ent,
                      cudaStream_t s);
@@ -100,11 +101,11 @@ int launch_rekey(int dim, int prec, const StepArgs& a, cudaStream_t s);
 int launch_fill_u32(uint32_t* p, uint32_t n, uint32_t v, cudaStream_t s);
 int launch_set_state(DevStats* st, long long n, long long next_id, long long add_id, cudaStream_t s);
 int launch_cell_v(int dim, int prec, const double* V, const double* Vold, const int32_t* cd, int nC, int nD, void* Vc,
-                  void* dVc, double* Vcopy, cudaStream_t s);
+                  void* dVc, double* Vcopy, double* Va, cudaStream_t s);
 int launch_nonfinite(const double* v, size_t n, unsigned* flag, cudaStream_t s);
 int launch_cell_rec32(int dim, const double* V, const double* Vold, const int32_t* cd, const double* aff,
                       const float* jinv32, int nC, int nD, float* vrec, float* dvrec, double* Vcopy,
-                      cudaStream_t s);
+                      double* Va, cudaStream_t s);
 
 // window_f64.cu / window_f32.cu: the differentiated window (window.cuh)
 struct WinArgs;

@@ -165,22 +165,35 @@ __global__ void k_set_state(DevStats* st, long long n, long long next_id, long l
 // Per-cell copy of the nodal velocity (and V - Vold, deltaV of
 // src/pfem2particlehandler.cpp:120-124) for every cell vertex, padded to
 // VS components (FP64 form).
-// The staged copy of V (component-major, ncopy values) written by the kernel
-// that reads V first, so a step needs no separate copy.
-__device__ __forceinline__ void copy_v(const double* __restrict__ V, double* __restrict__ Vcopy, size_t ncopy)
+// The staged copies of V written by the kernel that reads V first, so a step
+// needs no separate copy: component-major (Vcopy), and one row of VS doubles
+// per DoF (Va), which the relocations and new particles gather from.
+template <int DIM>
+__device__ __forceinline__ void copy_v(const double* __restrict__ V, int nD, double* __restrict__ Vcopy,
+                                       double* __restrict__ Va)
 {
-    if (!Vcopy) return;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < ncopy; i += (size_t)gridDim.x * blockDim.x)
-        Vcopy[i] = V[i];
+    constexpr int VS = Dims<DIM>::VS;
+    if (!Va) return;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nD; j += gridDim.x * blockDim.x) {
+        double v[VS];
+#pragma unroll
+        for (int d = 0; d < VS; ++d) v[d] = d < DIM ? V[(size_t)d * nD + j] : 0.0;
+#pragma unroll
+        for (int d = 0; d < VS; d += 2)
+            *reinterpret_cast<double2*>(Va + (size_t)j * VS + d) = make_double2(v[d], v[d + 1]);
+        if (Vcopy)
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) Vcopy[(size_t)d * nD + j] = v[d];
+    }
 }
 
 template <int DIM, typename Real>
 __global__ void k_cell_v(const double* __restrict__ V, const double* __restrict__ Vold, const int32_t* __restrict__ cd,
                          int nC, int nD, Real* __restrict__ Vc, Real* __restrict__ dVc, double* __restrict__ Vcopy,
-                         size_t ncopy)
+                         double* __restrict__ Va)
 {
     pdl_entry();
-    copy_v(V, Vcopy, ncopy);
+    copy_v<DIM>(V, nD, Vcopy, Va);
     constexpr int NV = 1 << DIM, VS = Dims<DIM>::VS;
     const int total = nC * NV;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
@@ -244,7 +257,7 @@ __global__ void __launch_bounds__(REC_TILE, 4) k_cell_rec32(const double* __rest
                                                          const int32_t* __restrict__ cd, const double* __restrict__ aff,
                                                          const float* __restrict__ jinv32, int nC, int nD,
                                                          float* __restrict__ vrec, float* __restrict__ dvrec,
-                                                         double* __restrict__ Vcopy, size_t ncopy)
+                                                         double* __restrict__ Vcopy, double* __restrict__ Va)
 {
     constexpr int NV = 1 << DIM, F = Dims<DIM>::REC4 * 4, F4 = Dims<DIM>::REC4, AFF = Dims<DIM>::AFF;
     __shared__ __align__(16) float rec_s[2][REC_TILE * F];
@@ -316,7 +329,7 @@ __global__ void __launch_bounds__(REC_TILE, 4) k_cell_rec32(const double* __rest
         }
         __syncthreads();
     }
-    copy_v(V, Vcopy, ncopy);
+    copy_v<DIM>(V, nD, Vcopy, Va);
 }
 
 int grid_for(const void* k, int threads) { return occupancy_grid(k, threads); }
@@ -355,16 +368,15 @@ int launch_set_state(DevStats* st, long long n, long long next_id, long long add
 }
 
 int launch_cell_v(int dim, int prec, const double* V, const double* Vold, const int32_t* cd, int nC, int nD, void* Vc,
-                  void* dVc, double* Vcopy, cudaStream_t s)
+                  void* dVc, double* Vcopy, double* Va, cudaStream_t s)
 {
-    const size_t nc = Vcopy ? (size_t)dim * nD : 0;
     const int total = nC * (1 << dim);
     const int g = (total + 255) / 256 < 8192 ? (total + 255) / 256 : 8192;
     const int grid = g > 0 ? g : 1;
-    if (dim == 2 && prec == 0) return launch_pdl(k_cell_v<2, double>, grid, 256, 0, s, V, Vold, cd, nC, nD, (double*)Vc, (double*)dVc, Vcopy, nc);
-    if (dim == 3 && prec == 0) return launch_pdl(k_cell_v<3, double>, grid, 256, 0, s, V, Vold, cd, nC, nD, (double*)Vc, (double*)dVc, Vcopy, nc);
-    if (dim == 2) return launch_pdl(k_cell_v<2, float>, grid, 256, 0, s, V, Vold, cd, nC, nD, (float*)Vc, (float*)dVc, Vcopy, nc);
-    return launch_pdl(k_cell_v<3, float>, grid, 256, 0, s, V, Vold, cd, nC, nD, (float*)Vc, (float*)dVc, Vcopy, nc);
+    if (dim == 2 && prec == 0) return launch_pdl(k_cell_v<2, double>, grid, 256, 0, s, V, Vold, cd, nC, nD, (double*)Vc, (double*)dVc, Vcopy, Va);
+    if (dim == 3 && prec == 0) return launch_pdl(k_cell_v<3, double>, grid, 256, 0, s, V, Vold, cd, nC, nD, (double*)Vc, (double*)dVc, Vcopy, Va);
+    if (dim == 2) return launch_pdl(k_cell_v<2, float>, grid, 256, 0, s, V, Vold, cd, nC, nD, (float*)Vc, (float*)dVc, Vcopy, Va);
+    return launch_pdl(k_cell_v<3, float>, grid, 256, 0, s, V, Vold, cd, nC, nD, (float*)Vc, (float*)dVc, Vcopy, Va);
     return 1;
 }
 
@@ -393,13 +405,13 @@ int launch_nonfinite(const double* v, size_t n, unsigned* flag, cudaStream_t s)
 }
 
 int launch_cell_rec32(int dim, const double* V, const double* Vold, const int32_t* cd, const double* aff,
-                      const float* jinv32, int nC, int nD, float* vrec, float* dvrec, double* Vcopy, cudaStream_t s)
+                      const float* jinv32, int nC, int nD, float* vrec, float* dvrec, double* Vcopy, double* Va,
+                      cudaStream_t s)
 {
-    const size_t nc = Vcopy ? (size_t)dim * nD : 0;
     const int g = (nC + REC_TILE - 1) / REC_TILE;
     const int grid = g < 1 ? 1 : g;
-    if (dim == 2) return launch_pdl(k_cell_rec32<2>, grid, REC_TILE, 0, s, V, Vold, cd, aff, jinv32, nC, nD, vrec, dvrec, Vcopy, nc);
-    return launch_pdl(k_cell_rec32<3>, grid, REC_TILE, 0, s, V, Vold, cd, aff, jinv32, nC, nD, vrec, dvrec, Vcopy, nc);
+    if (dim == 2) return launch_pdl(k_cell_rec32<2>, grid, REC_TILE, 0, s, V, Vold, cd, aff, jinv32, nC, nD, vrec, dvrec, Vcopy, Va);
+    return launch_pdl(k_cell_rec32<3>, grid, REC_TILE, 0, s, V, Vold, cd, aff, jinv32, nC, nD, vrec, dvrec, Vcopy, Va);
     return 1;
 }
 

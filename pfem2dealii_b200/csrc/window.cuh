@@ -178,7 +178,7 @@ __device__ __forceinline__ bool win_relocate(const WinArgs& w, uint32_t& c, Real
         Vec<DIM> xo, ue;
 #pragma unroll
         for (int d = 0; d < DIM; ++d) xo.v[d] = (double)xi[d];
-        velocity_from_dofs<DIM>(a.mesh.cd, a.Vd, a.mesh.nD, c, xo.v, ue.v);
+        velocity_from_dofs<DIM>(a.mesh.cd, a.Va, c, xo.v, ue.v);
         const SearchOut so = a.mesh.all_affine ? fallback64<DIM, true>(a.mesh, c, xo, ue, a.pp.dtp)
                                                : fallback64<DIM, false>(a.mesh, c, xo, ue, a.pp.dtp);
         if (!(so.flags & SRCH_FOUND)) return false;
@@ -256,7 +256,7 @@ __global__ void k_win_init(WinArgs w, const double* __restrict__ v0)
 // states before every sub-step of the segment starting at k0 (and its end
 // state) are recorded: always in a replay, and in the forward's last segment.
 template <int DIM, typename Real, bool REPLAY>
-__global__ void __launch_bounds__(256) k_win_adv(WinArgs w, int k, int k0, int record)
+__global__ void __launch_bounds__(256) k_win_adv(const __grid_constant__ WinArgs w, int k, int k0, int record)
 {
     const WinView<DIM, Real> V = win_view<DIM, Real, REPLAY>(w);
     const int S = w.a.pp.S;
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(256) k_win_adv(WinArgs w, int k, int k0, int r
 // Step k, second kernel: the queued particles' relocations and remaining
 // sub-steps (relocating again whenever they leave a cell).
 template <int DIM, typename Real, bool REPLAY>
-__global__ void __launch_bounds__(128) k_win_cross(WinArgs w, int k, int k0, int record)
+__global__ void __launch_bounds__(128, DIM == 2 ? 6 : 4) k_win_cross(const __grid_constant__ WinArgs w, int k, int k0, int record)
 {
     const WinView<DIM, Real> V = win_view<DIM, Real, REPLAY>(w);
     const int S = w.a.pp.S;
@@ -473,31 +473,42 @@ __global__ void k_win_bwd_init(WinArgs w, double* __restrict__ g_v0)
     }
 }
 
-// Warp-cooperative add of each lane's NV x DIM values into acc[key * NV*DIM + m]:
-// lanes in order, one atomic per run of equal keys per value (lanes with
-// key LOST add nothing).  All 32 lanes call it.
+// Warp-cooperative add of each lane's NVD values into acc[key * NVD + m] and,
+// with `second`, of another NVD values into acc2: lanes in order, one atomic
+// per run of equal keys per value (lanes with key LOST add nothing).  Lane m
+// walks value m of both sets' 2 x NVD; the rows are 33 doubles apart, so the
+// walking lanes' reads meet no bank twice.  All 32 lanes call it.  (One pass
+// over both sets with padded rows in place of one per set at a stride of 32:
+// 640 -> 250 us of a Turek window's backward, 4 segments of 1.9 M particles.)
+constexpr int WF_ROW = 33;
 template <int NVD>
-__device__ __forceinline__ void warp_flush(double* buf, uint32_t* keys, uint32_t key, const double* vals,
-                                           double* acc)
+__device__ __forceinline__ void warp_flush(double* buf, uint32_t* keys, uint32_t key, const double* vals, double* acc,
+                                           bool second, const double* vals2, double* acc2)
 {
     const int lane = threadIdx.x & 31;
     keys[lane] = key;
 #pragma unroll
-    for (int m = 0; m < NVD; ++m) buf[m * 32 + lane] = vals[m];
+    for (int m = 0; m < NVD; ++m) buf[m * WF_ROW + lane] = vals[m];
+    if (second)
+#pragma unroll
+        for (int m = 0; m < NVD; ++m) buf[(NVD + m) * WF_ROW + lane] = vals2[m];
     __syncwarp();
-    if (lane < NVD) {
+    for (int m = lane; m < (second ? 2 * NVD : NVD); m += 32) {
+        double* dst = m < NVD ? acc + m : acc2 + (m - NVD);
         uint32_t cur = LOST;
         double s = 0.0;
+#pragma unroll 8
         for (int l = 0; l < 32; ++l) {
             const uint32_t k = keys[l];
+            const double v = buf[m * WF_ROW + l];
             if (k != cur) {
-                if (cur != LOST) atomicAdd(acc + (size_t)cur * NVD + lane, s);
+                if (cur != LOST) atomicAdd(dst + (size_t)cur * NVD, s);
                 cur = k;
                 s = 0.0;
             }
-            s = s + buf[lane * 32 + l];
+            s = s + v;
         }
-        if (cur != LOST) atomicAdd(acc + (size_t)cur * NVD + lane, s);
+        if (cur != LOST) atomicAdd(dst + (size_t)cur * NVD, s);
     }
     __syncwarp();
 }
@@ -552,14 +563,15 @@ struct ShapeF {
     }
 };
 
+// Latency-bound (two dependent loads and an FP64 chain per sub-step): 2D holds 5 blocks per SM (96 registers).
 template <int DIM, typename Real, bool AFF>
-__global__ void __launch_bounds__(128, 3) k_win_rev(WinArgs w, int j)
+__global__ void __launch_bounds__(128, DIM == 2 ? 5 : 3) k_win_rev(const __grid_constant__ WinArgs w, int j)
 {
     constexpr int NV = 1 << DIM, NVD = NV * DIM, VS = Dims<DIM>::VS;
-    __shared__ double fbuf_s[4][32 * NVD];
+    extern __shared__ __align__(16) double fbuf_s[];  // 4 warps x 2 NVD x WF_ROW
     __shared__ uint32_t fkey_s[4][32];
     const int warp = threadIdx.x >> 5;
-    double* fbuf = fbuf_s[warp];
+    double* fbuf = fbuf_s + warp * 2 * NVD * WF_ROW;
     uint32_t* fkey = fkey_s[warp];
     const int k0 = j * w.C, k1 = min(w.K, k0 + w.C), S = w.a.pp.S;
     const int tseg = (k1 - k0) * S;
@@ -619,13 +631,46 @@ __global__ void __launch_bounds__(128, 3) k_win_rev(WinArgs w, int j)
                 invert64<DIM>(Jb, Bi);
             }
         }
+        // The recorded states come PF sub-steps ahead: they stream from HBM, and a sub-step's work waits on them.
+        constexpr int PF = 2;
+        uint32_t pc[PF];
+        Real px[PF][DIM];
+#pragma unroll
+        for (int q = 0; q < PF; ++q) {
+            const int t = tseg - 1 - q;
+            pc[q] = LOST;
+            if (act && t >= 0) {
+                pc[q] = w.rec_cell[(size_t)t * w.n + p];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) px[q][d] = ldw<Real>(w.rec_xi[d], (size_t)t * w.n + p);
+            }
+        }
         for (int t = tseg - 1; t >= 0; --t) {
             if (!act) continue;
-            const size_t o = (size_t)t * w.n + p;
-            const uint32_t ca = w.rec_cell[o];
+            const uint32_t ca = pc[0];
             double xa[DIM], y[DIM];
 #pragma unroll
-            for (int d = 0; d < DIM; ++d) xa[d] = (double)ldw<Real>(w.rec_xi[d], o);
+            for (int d = 0; d < DIM; ++d) xa[d] = (double)px[0][d];
+#pragma unroll
+            for (int q = 0; q + 1 < PF; ++q) {
+                pc[q] = pc[q + 1];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) px[q][d] = px[q + 1][d];
+            }
+            if (t > 0 && pc[0] != ca) {  // the next cell's rows on their way to L1
+                prefetch_l1(w.Wcell + (size_t)pc[0] * NV * VS);
+                if constexpr (DIM == 3) prefetch_l1(w.Wcell + (size_t)pc[0] * NV * VS + 16);
+                if constexpr (!AFF) {
+                    prefetch_l1(m.cellX + (size_t)pc[0] * NV * DIM);
+                    if constexpr (DIM == 3) prefetch_l1(m.cellX + (size_t)pc[0] * NV * DIM + 16);
+                }
+            }
+            if (t >= PF) {
+                const size_t o = (size_t)(t - PF) * w.n + p;
+                pc[PF - 1] = w.rec_cell[o];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) px[PF - 1][d] = ldw<Real>(w.rec_xi[d], o);
+            }
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {  // y = J^-T g
                 double sy = 0.0;
@@ -723,8 +768,7 @@ __global__ void __launch_bounds__(128, 3) k_win_rev(WinArgs w, int j)
 #pragma unroll
             for (int d = 0; d < DIM; ++d) cv[i * DIM + d] = accN[i] * gv[d];
         const uint32_t key = act ? acc_c : LOST;
-        warp_flush<NVD>(fbuf, fkey, key, acc, w.gadv);
-        if (w.do_correct) warp_flush<NVD>(fbuf, fkey, key, cv, w.gdv);
+        warp_flush<NVD>(fbuf, fkey, key, acc, w.gadv, w.do_correct, cv, w.gdv);
         if (act)
 #pragma unroll
             for (int d = 0; d < DIM; ++d) w.gxi[(size_t)d * w.n + p] = g[d];
@@ -778,6 +822,16 @@ inline int win_forward_t(const WinArgs& w, cudaStream_t s)
     return n;
 }
 
+template <int DIM, typename Real, bool AFF>
+inline void win_rev_launch(const WinArgs& w, int j, cudaStream_t s)
+{
+    constexpr int smem = 4 * 2 * (1 << DIM) * DIM * WF_ROW * (int)sizeof(double);  // 17 KB in 2D, 51 KB in 3D
+    auto* kernel = k_win_rev<DIM, Real, AFF>;
+    static const cudaError_t sized = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    (void)sized;
+    kernel<<<occupancy_grid((const void*)kernel, 128, smem), 128, smem, s>>>(w, j);
+}
+
 // Segments in reverse: replay (recording) unless the record buffer holds the
 // segment already (rec_seg), then the reverse sweep.
 template <int DIM, typename Real>
@@ -790,10 +844,8 @@ inline int win_backward_t(const WinArgs& w, double* g_v0, int rec_seg, cudaStrea
         const int k0 = j * w.C, k1 = k0 + w.C < w.K ? k0 + w.C : w.K;
         if (j != rec_seg)
             for (int k = k0; k < k1; ++k) n += win_step<DIM, Real, true>(w, k, k0, 1, s);
-        if (w.a.mesh.all_affine)
-            k_win_rev<DIM, Real, true><<<win_grid(k_win_rev<DIM, Real, true>, 128), 128, 0, s>>>(w, j);
-        else
-            k_win_rev<DIM, Real, false><<<win_grid(k_win_rev<DIM, Real, false>, 128), 128, 0, s>>>(w, j);
+        if (w.a.mesh.all_affine) win_rev_launch<DIM, Real, true>(w, j, s);
+        else win_rev_launch<DIM, Real, false>(w, j, s);
         n += 1;
     }
     return n;
