@@ -484,6 +484,13 @@ __device__ __forceinline__ void count_one(const StepArgs& a, uint32_t c, int pe)
     atomicOr(a.cocc + (size_t)c * a.pp.occw + (pe >> 6), 1ull << (pe & 63));
 }
 
+// The advect pass takes the particles in chunks of ADV_CH, 256 threads to a
+// chunk, or, in small sets, in quarters of them, 128 threads each: more
+// blocks, and a thread takes one particle, not two one after the other
+// (channel of 26 k particles: advect 12 -> 9 us, with RK2 in FP64 25 -> 15).
+constexpr int ADV_SMALL_CH = ADV_CH / 4;
+constexpr int adv_threads(int ch) { return ch == ADV_CH ? 256 : 128; }
+
 // One chunk of particle state staged in shared memory by bulk copies.
 template <int DIM, typename Real, int CH>
 struct AdvStage {
@@ -543,15 +550,14 @@ struct ChunkTicket {
     uint32_t tk, cf, cl;
 };
 
-template <int CH>
-__device__ __forceinline__ void ticket_cells(const StepArgs& a, uint32_t n, ChunkTicket& t, bool recs)
+__device__ __forceinline__ void ticket_cells(const StepArgs& a, uint32_t n, ChunkTicket& t, int sh, bool recs)
 {
-    const uint32_t nchunks = (n + CH - 1) / CH;
     t.cf = 1u;
     t.cl = 0u;  // no range unless loaded
-    if (recs && t.tk < nchunks) {
-        t.cf = a.chunk_first[t.tk];
-        t.cl = t.tk + 1 < nchunks ? a.chunk_first[t.tk + 1] : (uint32_t)a.mesh.nC - 1;
+    const uint32_t k = t.tk >> sh;  // the recorded chunk that holds this piece of it
+    if (recs && k * ADV_CH < n) {
+        t.cf = a.chunk_first[k];
+        t.cl = (k + 1) * ADV_CH < n ? a.chunk_first[k + 1] : (uint32_t)a.mesh.nC - 1;
     }
 }
 
@@ -603,6 +609,8 @@ __device__ __forceinline__ void staged_loop(const StepArgs& a, AdvStage<DIM, Rea
 {
     __shared__ uint32_t tk[2];
     const uint32_t n = (uint32_t)a.stats->n_slots;
+    constexpr int sh = CH == ADV_CH ? 0 : 2;  // whole recorded chunks, or quarters of them
+    static_assert(CH << sh == ADV_CH, "CH divides the recorded chunks");
     const uint32_t nchunks = (n + CH - 1) / CH;
     const bool recs = rs != nullptr;
     ChunkTicket hand{0u, 1u, 0u};  // thread 0: the next chunk to stage
@@ -616,7 +624,7 @@ __device__ __forceinline__ void staged_loop(const StepArgs& a, AdvStage<DIM, Rea
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             ChunkTicket t{atomicAdd(&a.stats->adv_next, 1u), 1u, 0u};
-            ticket_cells<CH>(a, n, t, recs);
+            ticket_cells(a, n, t, sh, recs);
             tk[b] = t.tk;
             if (t.tk < nchunks) stage_chunk<DIM, Real, CH, RS>(a, st[b], &bar[b], t, n, recs ? rs + b : nullptr);
         }
@@ -636,7 +644,7 @@ __device__ __forceinline__ void staged_loop(const StepArgs& a, AdvStage<DIM, Rea
         }
         uint32_t after = 0;
         if (threadIdx.x == 0) {  // loads and a ticket in flight while the block works
-            ticket_cells<CH>(a, n, hand, recs);
+            ticket_cells(a, n, hand, sh, recs);
             after = hand.tk < nchunks ? atomicAdd(&a.stats->adv_next, 1u) : 0xffffffffu;
         }
         const uint32_t base = chunk * CH;
@@ -745,8 +753,6 @@ __device__ __forceinline__ int substeps64(const StepArgs& a, uint32_t c, int s0,
 
 constexpr uint32_t OWN_CELL = 0x80000000u;  // queued sub-step: the own cell's inverse map is still to be taken
 
-constexpr int ADV64_CH = ADV_CH;  // the chunks whose first cells the seed and write passes record
-
 // Two doubles from shared memory, read where written: the compiler would
 // otherwise keep a cell's 24 velocities in registers over the sub-steps and
 // spill (702 us against 344 for the duct's 7.0 M particles: with 107 KB of
@@ -774,17 +780,18 @@ __device__ __forceinline__ void velocity64_s(const double* V, const double* xi, 
     }
 }
 
-template <int DIM, bool RK, bool LIN>
-__global__ void __launch_bounds__(256, LIN ? 2 : 1) k_advect64(const __grid_constant__ StepArgs a)
+template <int DIM, bool RK, bool LIN, int CH>
+__global__ void __launch_bounds__(adv_threads(CH), (LIN ? 2 : 1) * 256 / adv_threads(CH))
+    k_advect64(const __grid_constant__ StepArgs a)
 {
     pdl_entry();
     extern __shared__ __align__(128) unsigned char adv_raw[];
     __shared__ uint64_t bar[2];
-    auto* st = reinterpret_cast<AdvStage<DIM, double, ADV64_CH>*>(adv_raw);
-    auto* rs = reinterpret_cast<AdvLin64Stage*>(adv_raw + 2 * sizeof(AdvStage<DIM, double, ADV64_CH>));
+    auto* st = reinterpret_cast<AdvStage<DIM, double, CH>*>(adv_raw);
+    auto* rs = reinterpret_cast<AdvLin64Stage*>(adv_raw + 2 * sizeof(AdvStage<DIM, double, CH>));
     const MeshDev& m = a.mesh;
     AdvCounters k;
-    staged_loop<DIM, double, ADV64_CH, AdvLin64Stage>(a, st, bar, [&](AdvStage<DIM, double, ADV64_CH>& sg, int sidx,
+    staged_loop<DIM, double, CH, AdvLin64Stage>(a, st, bar, [&](AdvStage<DIM, double, CH>& sg, int sidx,
                                                                       uint32_t t, uint32_t i, bool in) {
         const uint32_t c = in ? sg.cell[t] : HOLE;
         const bool act = c != HOLE && in;
@@ -1249,17 +1256,17 @@ __device__ __forceinline__ int substeps32(const StepArgs& a, uint32_t c, int s0,
     return substeps32<DIM, AFF, RK>(a, c, s0, xi, r);
 }
 
-template <int DIM, bool AFF, bool RK = false>
-__global__ void __launch_bounds__(256, AFF ? 4 : 3) k_advect32(StepArgs a)
+template <int DIM, bool AFF, bool RK, int CH>
+__global__ void __launch_bounds__(adv_threads(CH), (AFF ? 4 : 3) * 256 / adv_threads(CH)) k_advect32(StepArgs a)
 {
     pdl_entry();
     extern __shared__ __align__(128) unsigned char adv_raw[];
     __shared__ uint64_t bar[2];
-    auto* st = reinterpret_cast<AdvStage<DIM, float, ADV_CH>*>(adv_raw);
-    auto* rs = reinterpret_cast<AdvRecStage<DIM>*>(adv_raw + 2 * sizeof(AdvStage<DIM, float, ADV_CH>));
+    auto* st = reinterpret_cast<AdvStage<DIM, float, CH>*>(adv_raw);
+    auto* rs = reinterpret_cast<AdvRecStage<DIM>*>(adv_raw + 2 * sizeof(AdvStage<DIM, float, CH>));
     const MeshDev& m = a.mesh;
     AdvCounters k;
-    staged_loop<DIM, float, ADV_CH>(a, st, bar, [&](AdvStage<DIM, float, ADV_CH>& sg, int sidx, uint32_t t, uint32_t i,
+    staged_loop<DIM, float, CH>(a, st, bar, [&](AdvStage<DIM, float, CH>& sg, int sidx, uint32_t t, uint32_t i,
                                                     bool in) {
         const uint32_t c = in ? sg.cell[t] : HOLE;
         const bool act = c != HOLE && in;

@@ -48,17 +48,25 @@ static int smem_grid32(K kernel, int threads, int smem)
 
 // RK: the midpoint sub-step (params.integrator = PFEM2GPU_RK2), compiled as
 // its own kernels so that the Euler ones carry no trace of it.
+template <int DIM, bool RK, bool AFF>
+static int advect32_a(const StepArgs& a, cudaStream_t s)
+{
+    const auto smem = [](int stage) { return 2 * (stage + (int)sizeof(AdvRecStage<DIM>)); };
+    static const int grid = smem_grid32(k_advect32<DIM, AFF, RK, ADV_CH>, adv_threads(ADV_CH),
+                                        smem(sizeof(AdvStage<DIM, float, ADV_CH>)));
+    if (!small_advect(a, grid))
+        return launch_pdl(k_advect32<DIM, AFF, RK, ADV_CH>, grid, adv_threads(ADV_CH),
+                          smem(sizeof(AdvStage<DIM, float, ADV_CH>)), s, a);
+    static const int grid_s = smem_grid32(k_advect32<DIM, AFF, RK, ADV_SMALL_CH>, adv_threads(ADV_SMALL_CH),
+                                          smem(sizeof(AdvStage<DIM, float, ADV_SMALL_CH>)));
+    return launch_pdl(k_advect32<DIM, AFF, RK, ADV_SMALL_CH>, small_grid(a, grid_s, ADV_SMALL_CH), adv_threads(ADV_SMALL_CH),
+                      smem(sizeof(AdvStage<DIM, float, ADV_SMALL_CH>)), s, a);
+}
+
 template <int DIM, bool RK>
 static int advect32_t(const StepArgs& a, cudaStream_t s)
 {
-    const int smem = 2 * (int)(sizeof(AdvStage<DIM, float, ADV_CH>) + sizeof(AdvRecStage<DIM>));
-    if (a.mesh.all_affine) {
-        static const int grid = smem_grid32(k_advect32<DIM, true, RK>, 256, smem);
-        return launch_pdl(k_advect32<DIM, true, RK>, grid, 256, smem, s, a);
-    } else {
-        static const int grid = smem_grid32(k_advect32<DIM, false, RK>, 256, smem);
-        return launch_pdl(k_advect32<DIM, false, RK>, grid, 256, smem, s, a);
-    }
+    return a.mesh.all_affine ? advect32_a<DIM, RK, true>(a, s) : advect32_a<DIM, RK, false>(a, s);
 }
 
 template <int DIM, bool RK>

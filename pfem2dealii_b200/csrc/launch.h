@@ -29,6 +29,20 @@ inline int occupancy_grid(const void* kernel, int threads, size_t smem = 0)
     return g;
 }
 
+// Whether the advect pass takes quarter chunks: fewer than 4 whole chunks per
+// block of the whole-chunk grid at two particles per cell part.
+inline bool small_advect(const StepArgs& a, int grid)
+{
+    return 2ll * (a.cend - a.cbeg) * a.pp.npart < 4ll * grid * ADV_CH;
+}
+
+// Their grid: at most one block per quarter chunk of that many particles.
+inline int small_grid(const StepArgs& a, int grid, int chunk)
+{
+    const long long n = (2ll * (a.cend - a.cbeg) * a.pp.npart + chunk - 1) / chunk;
+    return n < 1 ? 1 : n < grid ? (int)n : grid;
+}
+
 // Launch with programmatic dependent launch (the kernel calls pdl_entry()
 // first): it may be scheduled while the previous kernel drains, which hides
 // the launch gap between the dependent kernels of a step.  Returns 1 (one

@@ -114,6 +114,32 @@ __global__ void __launch_bounds__(SB) k_slots_down(StepArgs a, const unsigned lo
     }
 }
 
+// Both passes in one block for meshes of a few tiles, where the second
+// kernel's launch and wait cost as much as the work.
+constexpr int SMALL_TILES = 8;
+__global__ void __launch_bounds__(SB) k_slots_small(StepArgs a)
+{
+    pdl_entry();
+    const uint32_t n = (uint32_t)a.mesh.nC;
+    unsigned long long v[SMALL_TILES * SI];
+#pragma unroll
+    for (int k = 0; k < SMALL_TILES * SI; ++k) {
+        const uint32_t c = k * SB + threadIdx.x;
+        v[k] = c < n ? cell_slot_word(a, c) : 0ull;
+    }
+    unsigned long long carry = 0;
+#pragma unroll
+    for (int k = 0; k < SMALL_TILES * SI; ++k) {
+        const uint32_t c = k * SB + threadIdx.x;
+        if ((uint32_t)(k * SB) >= n) break;
+        unsigned long long total;
+        const unsigned long long p = block_excl_scan<unsigned long long, SB>(v[k], total);
+        if (c < n) a.coff[c] = carry + p;
+        if (c == n - 1) a.coff[n] = carry + p + v[k];
+        carry += total;
+    }
+}
+
 // An uploaded particle set: every particle is an arrival of its cell (the old
 // ranges are empty), counted with its part.
 template <typename Real, int DIM>
@@ -339,6 +365,7 @@ int grid_for(const void* k, int threads) { return occupancy_grid(k, threads); }
 int launch_slots_scan(const StepArgs& a, unsigned long long* tiles, cudaStream_t s)
 {
     const uint32_t ntiles = ((uint32_t)a.mesh.nC + STILE - 1) / STILE;
+    if (ntiles <= SMALL_TILES) return launch_pdl(k_slots_small, 1, SB, 0, s, a);
     const int r0 = launch_pdl(k_slots_reduce, (int)ntiles, SB, 0, s, a, tiles);
     const int r1 = launch_pdl(k_slots_down, (int)ntiles, SB, 0, s, a, (const unsigned long long*)tiles);
     if (r0 < 0 || r1 < 0) return -1;

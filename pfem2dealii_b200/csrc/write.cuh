@@ -18,9 +18,9 @@
 // cells above 32, and sent cells above 96 to a path that counts positions
 // through global scratch.  A run settles near 1.9 particles per part (54 a
 // cell at 27 parts, 124 at 64), so those were the paths in use.  Measured,
-// before -> now: duct FP32 (7.0 M particles) 480 -> 199 us, FP64 940 -> 489;
-// cube FP32 (32 M) 8414 -> 917, 37^3 cube FP64 (6.2 M) 3253 -> 465; Turek
-// mesh FP32 (1.9 M) 291 -> 100, FP64 429 -> 162.  Now bound by instruction
+// before -> now: duct FP32 (7.0 M particles) 480 -> 199 us, FP64 940 -> 406;
+// cube FP32 (32 M) 8414 -> 917, 37^3 cube FP64 (6.2 M) 3253 -> 373; Turek
+// mesh FP32 (1.9 M) 291 -> 91, FP64 429 -> 140.  Now bound by instruction
 // issue and the latencies a tile waits on one after the other (its copies,
 // about a third of its time, five barriers): a tile's headers and first
 // arrivals are therefore copied while the tile before it is worked on, and
@@ -283,40 +283,46 @@ __device__ __forceinline__ void partial_pairs32(float (*tr)[TRW], bool active, c
     }
 }
 
-// FP64 partial sums of one cell, in particle order (as the oracle adds them),
-// without shared rows: lane = entry (vertex lane / 4, component lane % 4).
-// Four particles at a time: the four lanes of a vertex take its shape value
-// of one particle each and exchange them by shuffles, and every lane adds its
-// component of the four in order.  2D has 16 entries; the upper lanes repeat
-// the lower ones' work.  at(r) = the staged entry of the r-th particle.
-template <int DIM, int CAP, typename At>
-__device__ __forceinline__ double partial_seq64(const double (*xi)[CAP], const double (*v)[CAP], uint32_t fin, int lane,
-                                                At&& at)
+// FP64 partial sums of up to 32 particles, one per lane, added to acc in lane
+// order, as the oracle adds them (lane = entry): 16 rows of PW entries at a
+// time through shared memory.  5 instructions a particle; one lane per entry
+// that recomputes or shuffles the shape values takes 15 (duct write pass,
+// 7.0 M particles: 489 us against 406).
+template <int DIM>
+struct Rows64 {
+    static constexpr int W = DIM == 3 ? 34 : 18;  // 16-byte stores of 8 lanes meet no bank twice
+};
+template <int DIM>
+__device__ __forceinline__ void partial_rows64(double (*tr)[Rows64<DIM>::W], uint32_t rows, const double* xi,
+                                               const double* v, int lane, double& acc)
 {
-    const int iv = (lane >> 2) & ((1 << DIM) - 1), comp = lane & 3;
-    const double* vc = v[comp < DIM ? comp : 0];
-    double acc = 0.0;
-    auto group = [&](uint32_t r0, uint32_t n) {
-        const uint32_t own = at(r0 + comp < fin ? r0 + comp : r0);
-        double N = lag64(iv & 1, xi[0][own]);
-        N = N * lag64((iv >> 1) & 1, xi[1][own]);
-        if (DIM > 2) N = N * lag64((iv >> 2) & 1, xi[DIM - 1][own]);
-        double t[4];
+    constexpr int NV = 1 << DIM, PW = Dims<DIM>::PW;
+    double N[NV];
+    shape64<DIM>(xi, N);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const double Nj = __shfl_sync(0xffffffffu, N, (lane & ~3) | j);
-            const uint32_t e = __shfl_sync(0xffffffffu, own, (lane & ~3) | j);
-            t[j] = comp < DIM ? Nj * vc[e] : (comp == DIM ? Nj : 0.0);
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t n = rows > 16u * h ? (rows - 16u * h < 16u ? rows - 16u * h : 16u) : 0u;
+        if (n == 0) break;
+        if ((lane >> 4) == h && (uint32_t)lane < rows) {
+            double* t = tr[lane & 15];
+#pragma unroll
+            for (int iv = 0; iv < NV; ++iv) {
+                *reinterpret_cast<double2*>(t + iv * 4) = make_double2(N[iv] * v[0], N[iv] * v[1]);
+                *reinterpret_cast<double2*>(t + iv * 4 + 2) =
+                    DIM == 3 ? make_double2(N[iv] * v[DIM - 1], N[iv]) : make_double2(N[iv], 0.0);
+            }
         }
+        __syncwarp();
+        if (lane < PW) {
+            if (n == 16) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if ((uint32_t)j < n) acc = acc + t[j];
-    };
-    uint32_t r0 = 0;
-#pragma unroll 2
-    for (; r0 + 4 <= fin; r0 += 4) group(r0, 4);
-    if (r0 < fin) group(r0, fin - r0);
-    return acc;
+                for (int r = 0; r < 16; ++r) acc = acc + tr[r][lane];
+            } else {
+                for (uint32_t r = 0; r < n; ++r) acc = acc + tr[r][lane];
+            }
+        }
+        __syncwarp();
+    }
 }
 
 // Copies of a few bytes, global -> shared, that complete at async_wait.
@@ -376,11 +382,15 @@ struct __align__(128) WtTile {
             int cnt[WT_CNT];
             uint16_t meta[TCAP];  // arrivals, new particles, over-full parts: local cell << 8 | extended part
         };
-        Real tr[HX ? 1 : WtCfg<DIM, Real>::WARPS][HX ? 1 : 16][TRW];  // FP32 partial rows, 16 per warp (once placed)
+        // FP32 partial rows, 16 per warp (once placed)
+        Real tr[HX ? 1 : WtCfg<DIM, Real>::WARPS][HX ? 1 : 16][TRW];
     };
+    Real x[HX ? DIM : 1][HX ? TCAP : 4];  // FP64: the partial rows take the space up to its end
     Real xi[DIM][TCAP];
     Real v[DIM][TCAP];
-    Real x[HX ? DIM : 1][HX ? TCAP : 4];
+    using Row64 = double[16][Rows64<DIM>::W];
+    static_assert(!HX || 10 * TCAP + 4 * WT_CNT + DIM * TCAP * 8 >= (int)sizeof(Row64) * WtCfg<DIM, Real>::WARPS,
+                  "the rows fit where keys, ids, counters and positions were");
     uint16_t perm[TCAP];       // over-full parts' entries, then the entry of each new slot
     uint32_t mask[TCAP / 32];  // survivors
     WtHead hdr[2];             // this tile's cells and the next one's
@@ -458,13 +468,12 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
         if ((uint32_t)lane <= ncell) h.aoff[lane] = inc - na;
         if (lane == 0) w.ticket = tile;
     };
-    uint32_t tk = 0;  // (the header warp) the next tile
+    uint32_t tk = 0;  // (the header warp) the next tile: the block's own first, then drawn ones
     if (warp == HW) {
-        if (lane == 0) tk = atomicAdd(&a.stats->write_next, 2u);
+        fetch_head(w.hdr[0], blockIdx.x);
+        if (lane == 0) tk = gridDim.x + atomicAdd(&a.stats->write_next, 1u);
+        land_head(w.hdr[0], blockIdx.x);
         tk = __shfl_sync(0xffffffffu, tk, 0);
-        fetch_head(w.hdr[0], tk);
-        land_head(w.hdr[0], tk);
-        ++tk;
     }
     for (uint32_t hb = 0;; hb ^= 1u) {
         __syncthreads();
@@ -475,7 +484,7 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
         uint32_t tk2 = 0;
         if (warp == HW) {
             fetch_head(w.hdr[hb ^ 1u], tk);
-            if (lane == 0) tk2 = atomicAdd(&a.stats->write_next, 1u);
+            if (lane == 0) tk2 = gridDim.x + atomicAdd(&a.stats->write_next, 1u);
         }
         for (uint32_t cb = 0; cb < ncell;) {
             // the longest run of cells [cb, ce) that fits
@@ -764,10 +773,20 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                     uint32_t fin = __shfl_sync(0xffffffffu, c_nsurv, (int)(lc - cb)) + nseed;
                     fin = fin < ub ? fin : ub;
                     if constexpr (HX) {
-                        const double s = partial_seq64<DIM, TCAP>(w.xi, w.v, fin, lane,
-                                                                  [&](uint32_t r) { return (uint32_t)perm[r]; });
+                        auto* tr = reinterpret_cast<typename WtTile<DIM, Real>::Row64*>(&w)[warp];
+                        double acc = 0.0;
+                        for (uint32_t r0 = 0; r0 < fin; r0 += 32) {
+                            const uint32_t e = perm[r0 + lane < fin ? r0 + lane : r0];
+                            double xs[DIM], vs[DIM];
+#pragma unroll
+                            for (int d = 0; d < DIM; ++d) {
+                                xs[d] = w.xi[d][e];
+                                vs[d] = w.v[d][e];
+                            }
+                            partial_rows64<DIM>(tr, fin - r0 < 32u ? fin - r0 : 32u, xs, vs, lane, acc);
+                        }
                         if (lane < Dims<DIM>::PW)
-                            reinterpret_cast<double*>(a.partials)[(size_t)c * Dims<DIM>::PW + lane] = s;
+                            reinterpret_cast<double*>(a.partials)[(size_t)c * Dims<DIM>::PW + lane] = acc;
                     } else {
                         PartialAcc<Real> acc;
                         const uint32_t L = h.cs[lc + 1] - h.cs[lc], na = h.na[lc];
