@@ -34,6 +34,14 @@ struct SearchOut {
     uint32_t map_failures;
 };
 
+// 2D: does the cell's closed-form inverse decide (mild_quad64)?
+template <int DIM>
+__device__ __forceinline__ bool mild_cell(const MeshDev& m, uint32_t c)
+{
+    if constexpr (DIM == 2) return __ldg(m.mild + c) != 0;
+    else return false;
+}
+
 // inverse_map64 of cell c, out of line: for the points that locate_lin64
 // leaves undecided (within 1e-9 of a face, or far outside).
 template <int DIM>
@@ -82,7 +90,7 @@ __device__ __forceinline__ int candidate64(const MeshDev& m, uint32_t cand, cons
     } else {
         double X[1 << DIM][DIM];
         load_cell64<DIM>(m.cellX, cand, X);
-        return inverse_map64<DIM>(X, m.aff + (size_t)cand * Dims<DIM>::AFF, p, xi);
+        return inverse_map64<DIM>(X, m.aff + (size_t)cand * Dims<DIM>::AFF, p, xi, mild_cell<DIM>(m, cand));
     }
 }
 
@@ -294,7 +302,7 @@ __device__ __forceinline__ SearchOut fallback64_body(const MeshDev& m, uint32_t 
 #pragma unroll
     for (int d = 0; d < DIM; ++d) x[d] = x[d] + ue.v[d] * dtp;
     const int st = LIN ? inverse_affine64<DIM>(m.aff + (size_t)c * AFF, x, xin)
-                       : inverse_map64<DIM>(X, m.aff + (size_t)c * AFF, x, xin);
+                       : inverse_map64<DIM>(X, m.aff + (size_t)c * AFF, x, xin, mild_cell<DIM>(m, c));
     SearchOut out;
     out.cell = c;
     out.flags = 0;
@@ -382,7 +390,7 @@ __device__ __forceinline__ SearchOut fallback64_body(const MeshDev& m, uint32_t 
             sc = inverse_affine64<DIM>(m.aff + (size_t)cand * AFF, x, xc);
         } else {
             load_cell64<DIM>(m.cellX, cand, X);
-            sc = inverse_map64<DIM>(X, m.aff + (size_t)cand * AFF, x, xc);
+            sc = inverse_map64<DIM>(X, m.aff + (size_t)cand * AFF, x, xc, mild_cell<DIM>(m, cand));
         }
         if (sc) {
             out.map_failures++;
@@ -726,6 +734,7 @@ __device__ __forceinline__ int substeps64(const StepArgs& a, uint32_t c, int s0,
     const MeshDev& m = a.mesh;
     double X[NV][DIM];
     if constexpr (!LIN || RK) load_cell64<DIM>(m.cellX, c, X);
+    const bool mild = mild_cell<DIM>(m, c);
     int s = s0;
     for (; s < a.pp.S; ++s) {
         transport64<DIM, RK>(a, X, c, xi, u);
@@ -738,7 +747,7 @@ __device__ __forceinline__ int substeps64(const StepArgs& a, uint32_t c, int s0,
         int st;
         const double* ca = m.aff + (size_t)c * Dims<DIM>::AFF;
         if constexpr (LIN) st = inverse_lin64<DIM>(m, [=](int j) { return __ldg(ca + j); }, c, x, xin);
-        else st = inverse_map64<DIM>(X, ca, x, xin);
+        else st = inverse_map64<DIM>(X, ca, x, xin, mild);
         if (st) k.map_failures++;
         if (st == 0 && inside_unit<DIM>(xin)) {
 #pragma unroll

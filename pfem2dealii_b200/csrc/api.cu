@@ -31,6 +31,7 @@ struct pfem2gpu_handle {
     float* geo32 = nullptr;
     uint32_t* twisted = nullptr;  // cells whose map is not affine; 3D cells unfit for locate_lin64 (set by cell_setup)
     bool all_affine = false, lin64 = false;
+    uint8_t* mild = nullptr;  // 2D: cells whose closed-form inverse decides (mild_quad64)
     // velocities
     double *Vstage = nullptr, *Vstage2 = nullptr, *Vout = nullptr;
     double* Va = nullptr;  // the staged V, one row per DoF
@@ -216,6 +217,7 @@ StepArgs args(pfem2gpu_handle* h)
     a.mesh.nC = h->nC;
     a.mesh.all_affine = h->all_affine ? 1 : 0;
     a.mesh.lin64 = h->lin64 ? 1 : 0;
+    a.mesh.mild = h->mild;
     a.mesh.nV = h->nV;
     a.mesh.nD = h->nD;
     a.mesh.cv = h->cv;
@@ -978,7 +980,7 @@ int pfem2gpu_destroy(pfem2gpu_handle* h)
                     (void*)h->key, (void*)h->next, (void*)h->xtmp, (void*)h->head, (void*)h->cs0, (void*)h->cs1,
                     (void*)h->carr, (void*)h->carrs, (void*)h->ccount, (void*)h->cocc, (void*)h->cub, (void*)h->coff,
                     (void*)h->tiles64, (void*)h->gscr, (void*)h->jinv32, (void*)h->xq, (void*)h->nxq,
-                    (void*)h->vrec32, (void*)h->dvrec32, h->partials, (void*)h->stats, (void*)h->twisted})
+                    (void*)h->vrec32, (void*)h->dvrec32, h->partials, (void*)h->stats, (void*)h->twisted, (void*)h->mild})
         dfree(p);
     dfree(h->chunk_first);
     for (void* p : {(void*)h->ob_i, (void*)h->ob_c, (void*)h->ob_n, h->xbuf}) dfree(p);
@@ -1109,7 +1111,7 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
                      (void**)&h->Vout, (void**)&h->Vin, (void**)&h->Vc, (void**)&h->dVc, (void**)&h->head, (void**)&h->cs0,
                      (void**)&h->cs1, (void**)&h->carr, (void**)&h->carrs, (void**)&h->ccount, (void**)&h->cocc,
                      (void**)&h->cub, (void**)&h->coff, (void**)&h->tiles64, (void**)&h->jinv32, (void**)&h->vrec32,
-                     (void**)&h->dvrec32, (void**)&h->partials, (void**)&h->twisted}) {
+                     (void**)&h->dvrec32, (void**)&h->partials, (void**)&h->twisted, (void**)&h->mild}) {
         dfree(*p);
         *p = nullptr;
     }
@@ -1161,6 +1163,7 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
         CK(cudaMemsetAsync(h->dvrec32, 0, nc * rec * 4, h->stream));
     }
     CK(dalloc(&h->jinv32, nc * (dim == 3 ? 12 : 8)));
+    if (dim == 2) CK(dalloc(&h->mild, nc));
     CK(dalloc(&h->twisted, 2));
     CK(cudaMemsetAsync(h->twisted, 0, 8, h->stream));
     CK(cudaMalloc(&h->partials, nc * PW * esize(h)));
@@ -1176,7 +1179,7 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
     run(h, "cell_setup",
         [&] {
             return launch_cell_setup(dim, h->nC, h->verts, h->cv, h->cellX, h->aff, h->geo32, h->jinv32, h->twisted,
-                                     h->stream);
+                                     h->mild, h->stream);
         });
     uint32_t twisted[2] = {0, 0};
     CK(cudaMemcpyAsync(twisted, h->twisted, 8, cudaMemcpyDeviceToHost, h->stream));

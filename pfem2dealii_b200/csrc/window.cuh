@@ -104,6 +104,7 @@ __device__ __forceinline__ int win_incell(const WinArgs& w, uint32_t p, uint32_t
         constexpr int NV = 1 << DIM;
         double X[NV][DIM];
         load_cell64<DIM>(a.mesh.cellX, c, X);
+        const bool mild = mild_cell<DIM>(a.mesh, c);
         for (; s < S; ++s) {
             if (t0 >= 0) win_record<DIM, Real>(w, t0 + s, p, c, xi);
             double u[DIM], xin[DIM];
@@ -113,7 +114,7 @@ __device__ __forceinline__ int win_incell(const WinArgs& w, uint32_t p, uint32_t
                 const double st = u[d] * a.pp.dtp;
                 x[d] = x[d] + st;
             }
-            const int st = inverse_map64<DIM>(X, a.mesh.aff + (size_t)c * Dims<DIM>::AFF, x, xin);
+            const int st = inverse_map64<DIM>(X, a.mesh.aff + (size_t)c * Dims<DIM>::AFF, x, xin, mild);
             if (!(st == 0 && inside_unit<DIM>(xin))) break;
 #pragma unroll
             for (int d = 0; d < DIM; ++d) xi[d] = xin[d];
