@@ -45,6 +45,11 @@ __device__ __forceinline__ void shape_grad64(const double* xi, double (*G)[DIM])
         }
 }
 
+// The sums of products here start with their first product, as a rounded one
+// that is never contracted into the next: what a start from zero gives, a
+// zero's sign in sums of nothing but zeros apart (coordinates of -0.0).  18
+// FP64 additions less in each Newton iteration (advect of the 37^3 cube's
+// 6.3 M particles 1938 -> 1862 us).
 template <int DIM>
 __device__ __forceinline__ void fwd64(const double (*X)[DIM], const double* xi, double* x)
 {
@@ -52,9 +57,9 @@ __device__ __forceinline__ void fwd64(const double (*X)[DIM], const double* xi, 
     shape64<DIM>(xi, N);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
-        double acc = 0.0;
+        double acc = __dmul_rn(N[0], X[0][d]);
 #pragma unroll
-        for (int i = 0; i < (1 << DIM); ++i) acc = acc + N[i] * X[i][d];
+        for (int i = 1; i < (1 << DIM); ++i) acc = acc + N[i] * X[i][d];
         x[d] = acc;
     }
 }
@@ -77,9 +82,9 @@ __device__ __forceinline__ void jac64(const double (*X)[DIM], const double* xi, 
     for (int d = 0; d < DIM; ++d)
 #pragma unroll
         for (int k = 0; k < DIM; ++k) {
-            double acc = 0.0;
+            double acc = __dmul_rn(G[0][k], X[0][d]);
 #pragma unroll
-            for (int i = 0; i < (1 << DIM); ++i) acc = acc + G[i][k] * X[i][d];
+            for (int i = 1; i < (1 << DIM); ++i) acc = acc + G[i][k] * X[i][d];
             J[d][k] = acc;
         }
 }
@@ -120,9 +125,9 @@ __device__ __forceinline__ void matvec64(const double (*A)[DIM], const double* x
 {
 #pragma unroll
     for (int k = 0; k < DIM; ++k) {
-        double acc = 0.0;
+        double acc = __dmul_rn(A[k][0], x[0]);
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) acc = acc + A[k][d] * x[d];
+        for (int d = 1; d < DIM; ++d) acc = acc + A[k][d] * x[d];
         y[k] = acc;
     }
 }
@@ -130,9 +135,9 @@ __device__ __forceinline__ void matvec64(const double (*A)[DIM], const double* x
 template <int DIM>
 __device__ __forceinline__ double norm2_64(const double* a)
 {
-    double s = 0.0;
+    double s = __dmul_rn(a[0], a[0]);
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) s = s + a[d] * a[d];
+    for (int d = 1; d < DIM; ++d) s = s + a[d] * a[d];
     return s;
 }
 
@@ -359,6 +364,8 @@ __device__ __forceinline__ int inverse_map64(const double (*X)[DIM], const doubl
         for (int d = 0; d < DIM; ++d) r[d] = p[d] - row[DIM * DIM + d];
         matvec64<DIM>(Ai, r, xi);
     }
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) xi[d] = 0.0 + xi[d];  // never -0: the Newton updates keep that
 #pragma unroll
     for (int d = 0; d < DIM; ++d) xi[d] = xi[d] < 0.0 ? 0.0 : (xi[d] > 1.0 ? 1.0 : xi[d]);
     fwd64<DIM>(X, xi, x);
