@@ -492,10 +492,11 @@ __device__ __forceinline__ void count_one(const StepArgs& a, uint32_t c, int pe)
     atomicOr(a.cocc + (size_t)c * a.pp.occw + (pe >> 6), 1ull << (pe & 63));
 }
 
-// The advect pass takes the particles in chunks of ADV_CH, 256 threads to a
-// chunk, or, in small sets, in quarters of them, 128 threads each: more
-// blocks, and a thread takes one particle, not two one after the other
-// (channel of 26 k particles: advect 12 -> 9 us, with RK2 in FP64 25 -> 15).
+// The FP32 form's advect pass takes the particles in chunks of ADV_CH, 256
+// threads to a chunk, or, in small sets, in quarters of them, 128 threads
+// each: more blocks, and a thread takes one particle, not two one after the
+// other (channel of 26 k particles: advect 12 -> 9 us).  The FP64 form takes
+// quarters always (adv64_blocks; the channel with RK2 25 -> 15 us).
 constexpr int ADV_SMALL_CH = ADV_CH / 4;
 constexpr int adv_threads(int ch) { return ch == ADV_CH ? 256 : 128; }
 
@@ -531,8 +532,9 @@ struct AdvRecStage {
 // V - Vold) and the affine inverses of the chunk's cells.  The loads of these
 // (24 + 24 + 12 doubles a particle, the first 24 in every sub-step) from
 // global memory held every warp for 4 of its 11 cycles per instruction.
+// MAXC cells hold a chunk of 128 particles from 18 to a cell on.
 struct __align__(16) AdvLin64Stage {
-    static constexpr int MAXC = 24, VW = 32, AW = 12;
+    static constexpr int MAXC = 8, VW = 32, AW = 12;
     double v[MAXC][VW];
     double dv[MAXC][VW];
     double aff[MAXC][AW];
@@ -558,14 +560,15 @@ struct ChunkTicket {
     uint32_t tk, cf, cl;
 };
 
-__device__ __forceinline__ void ticket_cells(const StepArgs& a, uint32_t n, ChunkTicket& t, int sh, bool recs)
+template <int CH>
+__device__ __forceinline__ void ticket_cells(const StepArgs& a, uint32_t n, ChunkTicket& t, bool recs)
 {
+    static_assert(CH % ADV_REC == 0, "a chunk starts at a recorded slot");
     t.cf = 1u;
     t.cl = 0u;  // no range unless loaded
-    const uint32_t k = t.tk >> sh;  // the recorded chunk that holds this piece of it
-    if (recs && k * ADV_CH < n) {
-        t.cf = a.chunk_first[k];
-        t.cl = (k + 1) * ADV_CH < n ? a.chunk_first[k + 1] : (uint32_t)a.mesh.nC - 1;
+    if (recs && t.tk * CH < n) {
+        t.cf = a.chunk_first[t.tk * (CH / ADV_REC)];
+        t.cl = (t.tk + 1) * CH < n ? a.chunk_first[(t.tk + 1) * (CH / ADV_REC)] : (uint32_t)a.mesh.nC - 1;
     }
 }
 
@@ -617,8 +620,6 @@ __device__ __forceinline__ void staged_loop(const StepArgs& a, AdvStage<DIM, Rea
 {
     __shared__ uint32_t tk[2];
     const uint32_t n = (uint32_t)a.stats->n_slots;
-    constexpr int sh = CH == ADV_CH ? 0 : 2;  // whole recorded chunks, or quarters of them
-    static_assert(CH << sh == ADV_CH, "CH divides the recorded chunks");
     const uint32_t nchunks = (n + CH - 1) / CH;
     const bool recs = rs != nullptr;
     ChunkTicket hand{0u, 1u, 0u};  // thread 0: the next chunk to stage
@@ -632,7 +633,7 @@ __device__ __forceinline__ void staged_loop(const StepArgs& a, AdvStage<DIM, Rea
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             ChunkTicket t{atomicAdd(&a.stats->adv_next, 1u), 1u, 0u};
-            ticket_cells(a, n, t, sh, recs);
+            ticket_cells<CH>(a, n, t, recs);
             tk[b] = t.tk;
             if (t.tk < nchunks) stage_chunk<DIM, Real, CH, RS>(a, st[b], &bar[b], t, n, recs ? rs + b : nullptr);
         }
@@ -652,7 +653,7 @@ __device__ __forceinline__ void staged_loop(const StepArgs& a, AdvStage<DIM, Rea
         }
         uint32_t after = 0;
         if (threadIdx.x == 0) {  // loads and a ticket in flight while the block works
-            ticket_cells(a, n, hand, sh, recs);
+            ticket_cells<CH>(a, n, hand, recs);
             after = hand.tk < nchunks ? atomicAdd(&a.stats->adv_next, 1u) : 0xffffffffu;
         }
         const uint32_t base = chunk * CH;
@@ -764,8 +765,9 @@ constexpr uint32_t OWN_CELL = 0x80000000u;  // queued sub-step: the own cell's i
 
 // Two doubles from shared memory, read where written: the compiler would
 // otherwise keep a cell's 24 velocities in registers over the sub-steps and
-// spill (702 us against 344 for the duct's 7.0 M particles: with 107 KB of
-// shared memory per block, spilled registers miss the small L1 that is left).
+// spill (702 us against 344 for the duct's 7.0 M particles, in blocks of 256:
+// with 200 KB of shared memory in use, spilled registers miss the small L1
+// that is left).
 __device__ __forceinline__ double2 lds2(const double* p)
 {
     double2 t;
@@ -789,10 +791,30 @@ __device__ __forceinline__ void velocity64_s(const double* V, const double* xi, 
     }
 }
 
-template <int DIM, bool RK, bool LIN, int CH>
-__global__ void __launch_bounds__(adv_threads(CH), (LIN ? 2 : 1) * 256 / adv_threads(CH))
+// Blocks of the FP64 advect pass on an SM.  Newton and the closed forms are
+// long chains of FP64 operations: warps in flight hide them, registers that
+// spill cost less.  With Newton, blocks of 128 threads (quarter chunks) for
+// any number of particles: 4 of them at 128 registers take 1449 us for the
+// 37^3 cube's 6.3 M particles, 3 at 164 without a spill 1478, one of 256
+// threads at 164 took 1862, two at 128 1525; the cells' rows staged in shared
+// memory and read at each use, 3 / 4 / 5 / 6 blocks, 1554 / 1493 / 1501 /
+// 1444.  Quads (Turek mesh, 1.9 M): 6 at 80 registers 129 us, two of 256
+// threads at 124 took 149, three at 80 131, staged rows 134 or more.  Affine
+// hexes (duct, 7.0 M): 7 at 72 registers 288 us, 6 at 80 304, two of 256
+// threads at 114 took 345; 8 at 64 would take 283, with room for 6 cells in
+// a stage, too few for chunks of freshly seeded cells.  The midpoint rule's
+// kernels keep the registers they need.
+template <int DIM, bool RK, bool LIN>
+constexpr int adv64_blocks()
+{
+    return RK ? (LIN ? 4 : 1) : LIN ? 7 : DIM == 2 ? 6 : 4;
+}
+
+template <int DIM, bool RK, bool LIN>
+__global__ void __launch_bounds__(adv_threads(ADV_SMALL_CH), adv64_blocks<DIM, RK, LIN>())
     k_advect64(const __grid_constant__ StepArgs a)
 {
+    constexpr int CH = ADV_SMALL_CH;
     pdl_entry();
     extern __shared__ __align__(128) unsigned char adv_raw[];
     __shared__ uint64_t bar[2];
@@ -887,7 +909,7 @@ __global__ void __launch_bounds__(adv_threads(CH), (LIN ? 2 : 1) * 256 / adv_thr
         }
         // a point that locate_lin64 leaves undecided is mapped by k_search64: the function calls of
         // inverse_map64 here would spill the loop's registers (684 against 344 us
-        // for the duct's 7.0 M particles)
+        // for the duct's 7.0 M particles, in blocks of 256)
         defer(a, want, i, where == 2 ? s | (int)OWN_CELL : s);
         count_cells(a, counted, c, pe);
     }, LIN && a.chunk_first ? rs : nullptr);

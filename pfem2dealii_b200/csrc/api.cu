@@ -51,7 +51,7 @@ struct pfem2gpu_handle {
     uint32_t *carr = nullptr, *carrs = nullptr, *ccount = nullptr;
     unsigned long long *cocc = nullptr, *cub = nullptr, *coff = nullptr, *tiles64 = nullptr;
     uint4* gscr = nullptr;
-    uint32_t* chunk_first = nullptr;  // first cell of each advect chunk of the current layout
+    uint32_t* chunk_first = nullptr;  // first cell of every ADV_REC slots of the current layout
     float *jinv32 = nullptr, *vrec32 = nullptr, *dvrec32 = nullptr;
     bool launch_failed = false;
     // CUDA graphs of the per-step sequences (one per buffer parity and
@@ -380,10 +380,10 @@ int ensure_capacity(pfem2gpu_handle* h, uint64_t need, uint64_t want = 0)
     CK(alloc_state(h, n1, (uint32_t)cap, true));
     CK(alloc_state(h, nt, (uint32_t)cap, false));
     uint32_t* cf_new = nullptr;
-    const size_t ncf = (cap + ADV_CH - 1) / ADV_CH + 1;
+    const size_t ncf = (cap + ADV_REC - 1) / ADV_REC + 1;
     CK(dalloc(&cf_new, ncf));
     if (h->chunk_first)
-        CK(cudaMemcpyAsync(cf_new, h->chunk_first, ((size_t)h->cap + ADV_CH - 1) / ADV_CH * 4 + 4,
+        CK(cudaMemcpyAsync(cf_new, h->chunk_first, ((size_t)h->cap + ADV_REC - 1) / ADV_REC * 4 + 4,
                            cudaMemcpyDeviceToDevice, h->stream));
     if (h->S0.cell && h->has_particles) {
         const size_t n = h->cap, es = esize(h);

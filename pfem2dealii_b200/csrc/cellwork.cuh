@@ -129,7 +129,7 @@ __global__ void k_seed(StepArgs a, uint32_t* cell_start)
         part_digits<DIM>(k, a.pp, idx);
         new_particle<DIM, Real>(a, a.S0, t, c, idx, id0 + t + 1);
         if (k == 0) cell_start[c] = t;
-        if (a.chunk_first && t % ADV_CH == 0) a.chunk_first[t / ADV_CH] = c;
+        if (a.chunk_first && t % ADV_REC == 0) a.chunk_first[t / ADV_REC] = c;
     }
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < (uint32_t)a.mesh.nC; c += gridDim.x * blockDim.x)
         if (c < cb || c >= ce) cell_start[c] = c < cb ? 0u : total;

@@ -23,6 +23,7 @@ constexpr int OCCW_MAX = 4;    // 64-bit part-occupancy words per cell
 constexpr int ARRCAP = 32;     // arrival slots per cell before the overflow list
 constexpr int CELL_WARPS = 4;  // warps per block of the warp-per-cell helper kernels
 constexpr int ADV_CH = 512;    // particles per staged chunk of the advect pass
+constexpr int ADV_REC = 128;   // slots per recorded first cell (chunk_first); a whole number of them to a chunk
 // cells whose velocity records an FP32 advect chunk stages with its particles
 // (a chunk spans about ADV_CH / particles-per-cell + 1 cells; beyond this
 // many, the chunk's particles read their records from global memory)
@@ -123,7 +124,7 @@ struct StepArgs {
     unsigned long long* cocc;  // nC x occw: parts occupied after the move
     unsigned long long* cub;   // nC: new particles << 32 | slots needed
     unsigned long long* coff;  // nC + 1: exclusive scan of cub
-    uint32_t* chunk_first;     // per ADV_CH-slot chunk of the layout the step writes: the cell its first slot
+    uint32_t* chunk_first;     // per ADV_REC slots of the layout the step writes: the cell its first slot
                                // belongs to (the seed and write passes fill it; null: not kept)
     const uint32_t* cs_old;    // nC + 1: cell ranges of S0
     uint32_t* cs_new;          // nC + 1: cell ranges of S1

@@ -126,16 +126,9 @@ static int smem_grid(K kernel, int threads, int smem)
 template <int DIM, bool RK, bool LIN>
 static int advect_l(const StepArgs& a, cudaStream_t s)
 {
-    const auto smem = [](int stage) { return 2 * (stage + (LIN ? (int)sizeof(AdvLin64Stage) : 0)); };
-    static const int grid = smem_grid(k_advect64<DIM, RK, LIN, ADV_CH>, adv_threads(ADV_CH),
-                                      smem(sizeof(AdvStage<DIM, double, ADV_CH>)));
-    if (!small_advect(a, grid))
-        return launch_pdl(k_advect64<DIM, RK, LIN, ADV_CH>, grid, adv_threads(ADV_CH),
-                          smem(sizeof(AdvStage<DIM, double, ADV_CH>)), s, a);
-    static const int grid_s = smem_grid(k_advect64<DIM, RK, LIN, ADV_SMALL_CH>, adv_threads(ADV_SMALL_CH),
-                                        smem(sizeof(AdvStage<DIM, double, ADV_SMALL_CH>)));
-    return launch_pdl(k_advect64<DIM, RK, LIN, ADV_SMALL_CH>, small_grid(a, grid_s, ADV_SMALL_CH), adv_threads(ADV_SMALL_CH),
-                      smem(sizeof(AdvStage<DIM, double, ADV_SMALL_CH>)), s, a);
+    constexpr int smem = 2 * (int)(sizeof(AdvStage<DIM, double, ADV_SMALL_CH>) + (LIN ? sizeof(AdvLin64Stage) : 0));
+    static const int grid = smem_grid(k_advect64<DIM, RK, LIN>, adv_threads(ADV_SMALL_CH), smem);
+    return launch_pdl(k_advect64<DIM, RK, LIN>, small_grid(a, grid, ADV_SMALL_CH), adv_threads(ADV_SMALL_CH), smem, s, a);
 }
 
 template <int DIM, bool RK>

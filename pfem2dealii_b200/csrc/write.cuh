@@ -204,13 +204,13 @@ __device__ __noinline__ uint2 write_cell_general(const StepArgs& a, int* cnt, Re
 }
 
 // A cell's new range [off, off + ub), within the capacity, and the advect
-// chunks that start in it.
+// chunks' recorded slots (ADV_REC) in it.
 __device__ __forceinline__ void new_range(const StepArgs& a, uint32_t c, uint32_t off, uint32_t ub)
 {
     const uint32_t first = off < a.capacity ? off : a.capacity, end = ub < a.capacity - first ? first + ub : a.capacity;
     a.cs_new[c] = first;
     if (a.chunk_first)
-        for (uint32_t k = (first + ADV_CH - 1) / ADV_CH; (uint64_t)k * ADV_CH < end; ++k) a.chunk_first[k] = c;
+        for (uint32_t k = (first + ADV_REC - 1) / ADV_REC; (uint64_t)k * ADV_REC < end; ++k) a.chunk_first[k] = c;
 }
 
 // FP32 partial sums of up to 32 particles, one per lane (lanes without a
