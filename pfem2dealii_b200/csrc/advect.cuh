@@ -917,9 +917,12 @@ __global__ void __launch_bounds__(adv_threads(ADV_SMALL_CH), adv64_blocks<DIM, R
 }
 
 // Deferred FP64 particles: the search of sub-step s (:438-491), then the
-// remaining sub-steps (searching again whenever needed).
+// remaining sub-steps (searching again whenever needed).  Bound by the latency
+// of its gathers: in 2D 6 blocks on an SM at 80 registers (Turek mesh, 412 k
+// crossings: 85 us, 5 87, 4 at 118 registers 93); in 3D 2 at 218 (duct 72, 4
+// at 128 89; cube 54 and 70).
 template <int DIM, bool RK, bool LIN>
-__global__ void __launch_bounds__(128) k_search64(const __grid_constant__ StepArgs a)
+__global__ void __launch_bounds__(128, DIM == 3 ? 2 : RK ? 4 : 6) k_search64(const __grid_constant__ StepArgs a)
 {
     pdl_entry();
     const uint32_t nq = *a.nxq < a.capacity ? *a.nxq : a.capacity;

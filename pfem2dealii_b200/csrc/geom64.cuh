@@ -330,7 +330,7 @@ __device__ __forceinline__ bool mild_quad64(const double (*X)[2], const double* 
 // Newton iterations (two thirds of a warp's FP64 operations where one lane
 // in five crosses a face) only told that the point is outside.  Turek mesh,
 // 1.9 M particles, 412 k crossings a step: advect of the FP64 form 201 -> 149
-// us, relocation of the FP32 form 83 -> 76, of the FP64 form 99 -> 93.
+// us, relocation of the FP32 form 83 -> 76, of the FP64 form 99 -> 93 (85 now).
 template <int DIM>
 __device__ __forceinline__ int inverse_map64(const double (*X)[DIM], const double* __restrict__ aff,
                                              const double* p, double* xi_out, bool mild = false)
