@@ -369,6 +369,7 @@ struct __align__(16) WtHead {
     uint32_t cs[WT_CELLS + 1];       // old slots
     uint32_t na[WT_CELLS];           // arrivals
     uint32_t aoff[WT_CELLS + 1];     // and their offsets in the tile
+    uint32_t tile;                   // written while other warps may still read the header before it
 };
 
 template <int DIM, typename Real>
@@ -395,7 +396,7 @@ struct __align__(128) WtTile {
     uint32_t mask[TCAP / 32];  // survivors
     WtHead hdr[2];             // this tile's cells and the next one's
     uint64_t bar;
-    uint32_t ticket, nover;
+    uint32_t nover;
 };
 
 template <int DIM, typename Real>
@@ -466,7 +467,7 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
             if (lane >= o) inc += y;
         }
         if ((uint32_t)lane <= ncell) h.aoff[lane] = inc - na;
-        if (lane == 0) w.ticket = tile;
+        if (lane == 0) h.tile = tile;
     };
     uint32_t tk = 0;  // (the header warp) the next tile: the block's own first, then drawn ones
     if (warp == HW) {
@@ -477,10 +478,10 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
     }
     for (uint32_t hb = 0;; hb ^= 1u) {
         __syncthreads();
-        const uint32_t tile = w.ticket;
+        const WtHead& h = w.hdr[hb];
+        const uint32_t tile = h.tile;
         if (tile >= ntiles) break;
         const uint32_t c0 = tile * NC, ncell = cells_of(tile);
-        const WtHead& h = w.hdr[hb];
         uint32_t tk2 = 0;
         if (warp == HW) {
             fetch_head(w.hdr[hb ^ 1u], tk);
