@@ -162,7 +162,7 @@ __device__ __noinline__ uint2 write_cell_general(const StepArgs& a, int* cnt, Re
         if (a.apply_counts && k > a.pp.maxpp + 1)
             for (uint32_t m = 0; m < n; ++m) {
                 const uint4 o = G[m];
-                rank += (o.y == g.y && o.z < g.z) ? 1 : 0;
+                rank += (o.y == g.y && (o.z < g.z || (o.z == g.z && o.x < g.x))) ? 1 : 0;
             }
         if (rank < survivors(k, a.pp.maxpp, a.apply_counts)) {
             G[e].w = g.w | 2u;
@@ -184,7 +184,8 @@ __device__ __noinline__ uint2 write_cell_general(const StepArgs& a, int* cnt, Re
             const uint4 o = G[m];
             if (!(o.w & 2u)) continue;
             const bool os = o.w & 1u;
-            pos += ((os && !gs) || (os && gs && o.x < g.x) || (!os && !gs && o.z < g.z)) ? 1u : 0u;
+            const bool less = os ? o.x < g.x : o.z < g.z || (o.z == g.z && o.x < g.x);
+            pos += ((os && !gs) || (os == gs && less)) ? 1u : 0u;
         }
         PData<DIM, Real> pd;
         load_global<DIM, Real>(a, g.x, pd);
@@ -378,7 +379,7 @@ struct __align__(128) WtTile {
     static constexpr int TCAP = WtCfg<DIM, Real>::TCAP;
     union {
         struct {
-            uint32_t key[TCAP];  // old slots: the move's cell; arrivals: key_of(id)
+            uint32_t key[TCAP];  // old slots: the move's cell; arrivals: key_of(id), the dead ones' ~0
             uint32_t id[TCAP];
             int cnt[WT_CNT];
             uint16_t meta[TCAP];  // arrivals, new particles, over-full parts: local cell << 8 | extended part
@@ -397,7 +398,100 @@ struct __align__(128) WtTile {
     WtHead hdr[2];             // this tile's cells and the next one's
     uint64_t bar;
     uint32_t nover;
+    int ties[2];  // below zero once equal keys share a rank: over-full parts, arrivals
 };
+
+// Equal keys (a caller's duplicate ids, or 32-bit ids that wrapped) go by the
+// particles' indices, so that every entry has a rank and a place of its own:
+// a place that two entries share would leave another without one, and the
+// partial sums would take what stands there for an entry.  The ranks of k
+// distinct keys add up to k (k - 1) / 2, those of equal ones to less: k_write
+// sums the difference over a run (a compare in its inner loops instead costs
+// 4 % of the FP32 pass) and calls these two, all threads together, where it
+// is not zero.
+template <int DIM, typename Real>
+__device__ __forceinline__ uint32_t entry_particle(const StepArgs& a, const WtHead& h, uint32_t c0, uint32_t lc,
+                                                   uint32_t SA, uint32_t nold, uint32_t a0, uint32_t e)
+{
+    if (e < nold) return SA + e;
+    const uint32_t k = e - nold - (h.aoff[lc] - a0);
+    if (k < (uint32_t)WT_ARR) return h.arr[lc][k];
+    if (k < (uint32_t)ARRCAP) return a.carrs[(size_t)(c0 + lc) * ARRCAP + k];
+    uint32_t p = a.head[c0 + lc];
+    for (uint32_t t = ARRCAP; t < k && p < a.capacity; ++t) p = a.next[p];
+    return p;
+}
+
+// Over-full entries (perm[0 .. nov)) that survive by their key but not by
+// their index; returns how many this thread took out.
+template <int DIM, typename Real>
+__device__ __noinline__ uint32_t ties_in_parts(const StepArgs& a, WtTile<DIM, Real>& w, uint32_t hb, uint32_t c0,
+                                               uint32_t cb, uint32_t ce, uint32_t nov)
+{
+    const WtHead& h = w.hdr[hb];
+    const uint32_t SA = h.cs[cb] & ~3u, nold = h.cs[cb] < h.cs[ce] ? ((h.cs[ce] + 3u) & ~3u) - SA : 0u;
+    uint32_t out = 0;
+    for (uint32_t j = threadIdx.x; j < nov; j += WtCfg<DIM, Real>::THREADS) {
+        const uint32_t e = w.perm[j], me = w.meta[e], lc = me >> 8, kk = key_of(w.id[e], a.pp.seed);
+        const uint32_t i = entry_particle<DIM, Real>(a, h, c0, lc, SA, nold, h.aoff[cb], e);
+        int rank = 0, before = 0;
+        for (uint32_t o = 0; o < nov; ++o) {
+            const uint32_t f = w.perm[o], kf = key_of(w.id[f], a.pp.seed);
+            if (w.meta[f] != me) continue;
+            rank += kf < kk ? 1 : 0;
+            before += kf == kk && entry_particle<DIM, Real>(a, h, c0, lc, SA, nold, h.aoff[cb], f) < i ? 1 : 0;
+        }
+        if (rank < a.pp.maxpp + 1 && rank + before >= a.pp.maxpp + 1) {
+            atomicAnd(w.mask + (e >> 5), ~(1u << (e & 31u)));
+            w.key[e] = ~0u;
+            out++;
+        }
+    }
+    __syncthreads();  // every thread has seen the count and the list
+    if (threadIdx.x == 0) w.ties[0] = 0;
+    return out;
+}
+
+// Arrivals of one key: the places after the first, and the first once more
+// (all of them were put there).
+template <int DIM, typename Real>
+__device__ __noinline__ void ties_in_cells(const StepArgs& a, WtTile<DIM, Real>& w, uint32_t hb, uint32_t c0,
+                                           uint32_t cb, uint32_t ce)
+{
+    const WtHead& h = w.hdr[hb];
+    const uint32_t SA = h.cs[cb] & ~3u, nold = h.cs[cb] < h.cs[ce] ? ((h.cs[ce] + 3u) & ~3u) - SA : 0u;
+    const uint32_t a0 = h.aoff[cb], nE = nold + h.aoff[ce] - a0, ob = h.co[cb].x;
+    auto live = [&](uint32_t e) { return (w.mask[e >> 5] >> (e & 31u)) & 1u; };
+    for (uint32_t e = nold + threadIdx.x; e < nE; e += WtCfg<DIM, Real>::THREADS) {
+        if (!live(e)) continue;
+        const uint32_t lc = w.meta[e] >> 8, o1 = nold + h.aoff[lc + 1] - a0;
+        const uint32_t i = entry_particle<DIM, Real>(a, h, c0, lc, SA, nold, a0, e);
+        uint32_t pos = 0, same = 0;
+        for (uint32_t o = nold + h.aoff[lc] - a0; o < o1; ++o) {
+            if (!live(o)) continue;
+            const bool eq = w.key[o] == w.key[e];
+            same += eq ? 1u : 0u;
+            pos += (w.key[o] < w.key[e] || (eq && entry_particle<DIM, Real>(a, h, c0, lc, SA, nold, a0, o) < i)) ? 1u : 0u;
+        }
+        if (same < 2) continue;
+        if (nold)
+            for (uint32_t o = h.cs[lc] - SA; o < h.cs[lc + 1] - SA; ++o) pos += live(o);
+        const uint32_t dst = h.co[lc].x + pos;
+        if (pos >= h.co[lc + 1].x - h.co[lc].x) continue;
+        w.perm[dst - ob] = (uint16_t)e;
+        if (dst >= a.capacity) continue;
+        a.S1.cell[dst] = c0 + lc;
+        a.S1.id[dst] = w.id[e];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            str<Real>(a.S1.xi[d], dst, w.xi[d][e]);
+            str<Real>(a.S1.v[d], dst, w.v[d][e]);
+            if constexpr (WtTile<DIM, Real>::HX) str<double>(a.S1.x[d], dst, w.x[d][e]);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) w.ties[1] = 0;
+}
 
 template <int DIM, typename Real>
 __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>::BLOCKS))
@@ -417,6 +511,7 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
         mbar_init(&w.bar, 1);
         mbar_fence_init();
         w.nover = 0;
+        w.ties[0] = w.ties[1] = 0;
     }
     pdl_entry();
     const uint32_t nC = (uint32_t)a.mesh.nC, cap = a.capacity;
@@ -621,7 +716,10 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                             }
                             done += __popc(b);
                         }
-                        if (done != n1) err |= ERR_COUNT;
+                        if (done != n1) {  // every entry has a cell all the same
+                            err |= ERR_COUNT;
+                            for (uint32_t j = done + lane; j < n1; j += 32) w.meta[nE + (sb - sb0) + j] = (uint16_t)(lc << 8);
+                        }
                     }
                 }
                 async_wait();
@@ -650,7 +748,7 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                         if (lc >= cb && lc < ce && slot >= h.cs[lc] && slot < h.cs[lc + 1]) m[r] = lc << 8;
                     } else if (e < nT) {
                         m[r] = w.meta[e];
-                        if (e < nE) w.key[e] = key_of(w.id[e], a.pp.seed);
+                        if (e < nE) w.key[e] = m[r] != NONE ? key_of(w.id[e], a.pp.seed) : ~0u;
                     }
                     if (e < nE && m[r] != NONE) {
                         Real xi[DIM];
@@ -679,17 +777,26 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                 }
                 if (__syncthreads_or(over)) {
                     const uint32_t nov = w.nover;
+                    int tie = 0;
                     for (uint32_t j = tid; j < nov; j += THREADS) {
                         const uint32_t e = w.perm[j], me = w.meta[e], kk = key_of(w.id[e], a.pp.seed);
                         int rank = 0;
                         for (uint32_t o = 0; o < nov; ++o) {
-                            const uint32_t f = w.perm[o];
-                            rank += (w.meta[f] == me && key_of(w.id[f], a.pp.seed) < kk) ? 1 : 0;
+                            const uint32_t f = w.perm[o], kf = key_of(w.id[f], a.pp.seed);
+                            rank += (w.meta[f] == me && kf < kk) ? 1 : 0;
                         }
-                        if (rank < maxpp + 1) atomicOr(w.mask + (e >> 5), 1u << (e & 31u));
-                        else removed++;
+                        tie += 2 * rank - (w.cnt[((me >> 8) - cb) * npe + (me & 255u)] - 1);
+                        if (rank < maxpp + 1) {
+                            atomicOr(w.mask + (e >> 5), 1u << (e & 31u));
+                        } else {
+                            w.key[e] = ~0u;
+                            removed++;
+                        }
                     }
+                    tie = __reduce_add_sync(0xffffffffu, tie);
+                    if (lane == 0 && tie) atomicAdd(&w.ties[0], tie);
                     __syncthreads();
+                    if (w.ties[0]) removed += ties_in_parts<DIM, Real>(a, w, hb, c0, cb, ce, nov);
                     if (tid == 0) w.nover = 0;
                 }
                 // survivors before an entry: words by a scan over the lanes, bits by a count
@@ -715,6 +822,7 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                     c_nsurv = c_ns + before(nold + h.aoff[lc + 1] - a0) - before(nold + h.aoff[lc] - a0);
                 }
                 // places and stores
+                int ties = 0;
 #pragma unroll
                 for (int r = 0; r < ROUNDS; ++r) {
                     const uint32_t e = r * THREADS + tid;
@@ -735,7 +843,8 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                         const uint32_t kk = w.key[e];
                         const uint32_t o1 = nold + h.aoff[lc + 1] - a0;
                         for (uint32_t o = nold + h.aoff[lc] - a0; o < o1; ++o)
-                            pos += (((w.mask[o >> 5] >> (o & 31u)) & 1u) && w.key[o] < kk) ? 1u : 0u;
+                            pos += w.key[o] < kk ? 1u : 0u;
+                        ties += 2 * (int)(pos - nst) - (int)(nsv - nst - 1u);
                     } else {
                         pos = nsv + (e - nE - (co.y - sb0));
                     }
@@ -765,8 +874,11 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                         if (j < cap) a.S1.cell[j] = HOLE;
                     new_range(a, c0 + cb + lane, co.x, cn.x - co.x);
                 }
+                ties = __reduce_add_sync(0xffffffffu, ties);
+                if (lane == 0 && ties) atomicAdd(&w.ties[1], ties);
                 __syncthreads();
-                // partial sums, a warp per cell
+                if (w.ties[1]) ties_in_cells<DIM, Real>(a, w, hb, c0, cb, ce);
+                // partial sums, a warp per cell; every place below a cell's count has its entry in perm
                 for (uint32_t lc = cb + warp; lc < ce; lc += WARPS) {
                     const uint32_t c = c0 + lc, ub = h.co[lc + 1].x - h.co[lc].x, nseed = h.co[lc + 1].y - h.co[lc].y;
                     const uint16_t* perm = w.perm + (h.co[lc].x - ob);
