@@ -327,9 +327,16 @@ __global__ void __launch_bounds__(256) k_win_adv(const __grid_constant__ WinArgs
 }
 
 // Step k, second kernel: the queued particles' relocations and remaining
-// sub-steps (relocating again whenever they leave a cell).
+// sub-steps (relocating again whenever they leave a cell).  2D: 6 blocks per
+// SM.  3D keeps its 198 to 209 registers: held to 4 blocks it spills them, and
+// those of the relocations it calls (cube of 30^3 cells, forward 1587 against
+// 1541 us).
+template <int DIM>
+struct WinCross {
+    static constexpr int BLOCKS = DIM == 2 ? 6 : 2;
+};
 template <int DIM, typename Real, bool REPLAY>
-__global__ void __launch_bounds__(128, DIM == 2 ? 6 : 4) k_win_cross(const __grid_constant__ WinArgs w, int k, int k0, int record)
+__global__ void __launch_bounds__(128, WinCross<DIM>::BLOCKS) k_win_cross(const __grid_constant__ WinArgs w, int k, int k0, int record)
 {
     const WinView<DIM, Real> V = win_view<DIM, Real, REPLAY>(w);
     const int S = w.a.pp.S;
@@ -477,31 +484,39 @@ __global__ void k_win_bwd_init(WinArgs w, double* __restrict__ g_v0)
 // Warp-cooperative add of each lane's NVD values into acc[key * NVD + m] and,
 // with `second`, of another NVD values into acc2: lanes in order, one atomic
 // per run of equal keys per value (lanes with key LOST add nothing).  Lane m
-// walks value m of both sets' 2 x NVD; the rows are 33 doubles apart, so the
-// walking lanes' reads meet no bank twice.  All 32 lanes call it.  (One pass
-// over both sets with padded rows in place of one per set at a stride of 32:
-// 640 -> 250 us of a Turek window's backward, 4 segments of 1.9 M particles.)
+// walks value m; the rows are 33 doubles apart, so the walking lanes' reads
+// meet no bank twice.  In 2D one pass takes both sets' 2 x 8 values; in 3D
+// one set's 24 fill a warp, and the sets go one after the other through half
+// the shared memory.  All 32 lanes call it.  (Padded rows and one pass in
+// place of two at a stride of 32: 640 -> 250 us of a Turek window's backward,
+// 4 segments of 1.9 M particles.)
 constexpr int WF_ROW = 33;
 template <int NVD>
+struct WinFlush {
+    static constexpr int SETS = 2 * NVD <= 32 ? 2 : 1;
+    static constexpr int ROWS = SETS * NVD;
+};
+template <int NVD>
 __device__ __forceinline__ void warp_flush(double* buf, uint32_t* keys, uint32_t key, const double* vals, double* acc,
-                                           bool second, const double* vals2, double* acc2)
+                                           bool second = false, const double* vals2 = nullptr, double* acc2 = nullptr)
 {
     const int lane = threadIdx.x & 31;
+    const bool two = WinFlush<NVD>::SETS == 2 && second;
     keys[lane] = key;
 #pragma unroll
     for (int m = 0; m < NVD; ++m) buf[m * WF_ROW + lane] = vals[m];
-    if (second)
+    if (two)
 #pragma unroll
         for (int m = 0; m < NVD; ++m) buf[(NVD + m) * WF_ROW + lane] = vals2[m];
     __syncwarp();
-    for (int m = lane; m < (second ? 2 * NVD : NVD); m += 32) {
-        double* dst = m < NVD ? acc + m : acc2 + (m - NVD);
+    if (lane < (two ? 2 * NVD : NVD)) {
+        double* dst = lane < NVD ? acc + lane : acc2 + (lane - NVD);
         uint32_t cur = LOST;
         double s = 0.0;
 #pragma unroll 8
         for (int l = 0; l < 32; ++l) {
             const uint32_t k = keys[l];
-            const double v = buf[m * WF_ROW + l];
+            const double v = buf[lane * WF_ROW + l];
             if (k != cur) {
                 if (cur != LOST) atomicAdd(dst + (size_t)cur * NVD, s);
                 cur = k;
@@ -564,15 +579,27 @@ struct ShapeF {
     }
 };
 
-// Latency-bound (two dependent loads and an FP64 chain per sub-step): 2D holds 5 blocks per SM (96 registers).
+// Latency-bound (two dependent loads and an FP64 chain per sub-step).  2D: 5
+// blocks per SM at 96 registers, the recorded states read two sub-steps ahead
+// (Turek mesh, 1.9 M particles: 797 -> 545 us a segment).  3D has no registers
+// left for states read ahead: the backward of a 64x20x20 duct (1.4 M, 10
+// steps) takes 1747 us in FP32 and 2779 in FP64 at 3 blocks and 168 registers
+// without them, 1905 and 2838 with one sub-step's, 2196 and 3134 with 2 blocks
+// and no spill; of a 30^3 cube 4273 us in FP64 (4348 with one ahead), and in
+// FP32 2323 at 4 blocks, 2482 at 3.
 template <int DIM, typename Real, bool AFF>
-__global__ void __launch_bounds__(128, DIM == 2 ? 5 : 3) k_win_rev(const __grid_constant__ WinArgs w, int j)
+struct WinRev {
+    static constexpr int BLOCKS = DIM == 2 ? 5 : std::is_same<Real, float>::value && !AFF ? 4 : 3;
+    static constexpr int PF = DIM == 2 ? 2 : 0;  // sub-steps read ahead
+};
+template <int DIM, typename Real, bool AFF>
+__global__ void __launch_bounds__(128, (WinRev<DIM, Real, AFF>::BLOCKS)) k_win_rev(const __grid_constant__ WinArgs w, int j)
 {
     constexpr int NV = 1 << DIM, NVD = NV * DIM, VS = Dims<DIM>::VS;
-    extern __shared__ __align__(16) double fbuf_s[];  // 4 warps x 2 NVD x WF_ROW
+    __shared__ double fbuf_s[4][WinFlush<NVD>::ROWS * WF_ROW];
     __shared__ uint32_t fkey_s[4][32];
     const int warp = threadIdx.x >> 5;
-    double* fbuf = fbuf_s + warp * 2 * NVD * WF_ROW;
+    double* fbuf = fbuf_s[warp];
     uint32_t* fkey = fkey_s[warp];
     const int k0 = j * w.C, k1 = min(w.K, k0 + w.C), S = w.a.pp.S;
     const int tseg = (k1 - k0) * S;
@@ -632,46 +659,37 @@ __global__ void __launch_bounds__(128, DIM == 2 ? 5 : 3) k_win_rev(const __grid_
                 invert64<DIM>(Jb, Bi);
             }
         }
-        // The recorded states come PF sub-steps ahead: they stream from HBM, and a sub-step's work waits on them.
-        constexpr int PF = 2;
-        uint32_t pc[PF];
-        Real px[PF][DIM];
+        // The recorded states stream from HBM and come PF sub-steps ahead, where there is room for them.
+        constexpr int PF = WinRev<DIM, Real, AFF>::PF, NEXT = PF > 0 ? PF - 1 : 0;
+        uint32_t pc[NEXT + 1];
+        Real px[NEXT + 1][DIM];
+        auto state = [&](int t, int q) {
+            const size_t o = (size_t)t * w.n + p;
+            pc[q] = w.rec_cell[o];
 #pragma unroll
-        for (int q = 0; q < PF; ++q) {
-            const int t = tseg - 1 - q;
-            pc[q] = LOST;
-            if (act && t >= 0) {
-                pc[q] = w.rec_cell[(size_t)t * w.n + p];
+            for (int d = 0; d < DIM; ++d) px[q][d] = ldw<Real>(w.rec_xi[d], o);
+        };
 #pragma unroll
-                for (int d = 0; d < DIM; ++d) px[q][d] = ldw<Real>(w.rec_xi[d], (size_t)t * w.n + p);
-            }
-        }
+        for (int q = 0; q < PF; ++q)
+            if (act && tseg - 1 - q >= 0) state(tseg - 1 - q, q);
         for (int t = tseg - 1; t >= 0; --t) {
             if (!act) continue;
+            if (PF == 0) state(t, 0);
             const uint32_t ca = pc[0];
             double xa[DIM], y[DIM];
 #pragma unroll
             for (int d = 0; d < DIM; ++d) xa[d] = (double)px[0][d];
 #pragma unroll
-            for (int q = 0; q + 1 < PF; ++q) {
+            for (int q = 0; q < NEXT; ++q) {
                 pc[q] = pc[q + 1];
 #pragma unroll
                 for (int d = 0; d < DIM; ++d) px[q][d] = px[q + 1][d];
             }
-            if (t > 0 && pc[0] != ca) {  // the next cell's rows on their way to L1
+            if (PF > 1 && t > 0 && pc[0] != ca) {  // the next cell's rows on their way to L1
                 prefetch_l1(w.Wcell + (size_t)pc[0] * NV * VS);
-                if constexpr (DIM == 3) prefetch_l1(w.Wcell + (size_t)pc[0] * NV * VS + 16);
-                if constexpr (!AFF) {
-                    prefetch_l1(m.cellX + (size_t)pc[0] * NV * DIM);
-                    if constexpr (DIM == 3) prefetch_l1(m.cellX + (size_t)pc[0] * NV * DIM + 16);
-                }
+                if constexpr (!AFF) prefetch_l1(m.cellX + (size_t)pc[0] * NV * DIM);
             }
-            if (t >= PF) {
-                const size_t o = (size_t)(t - PF) * w.n + p;
-                pc[PF - 1] = w.rec_cell[o];
-#pragma unroll
-                for (int d = 0; d < DIM; ++d) px[PF - 1][d] = ldw<Real>(w.rec_xi[d], o);
-            }
+            if (PF > 0 && t >= PF) state(t - PF, NEXT);
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {  // y = J^-T g
                 double sy = 0.0;
@@ -769,7 +787,12 @@ __global__ void __launch_bounds__(128, DIM == 2 ? 5 : 3) k_win_rev(const __grid_
 #pragma unroll
             for (int d = 0; d < DIM; ++d) cv[i * DIM + d] = accN[i] * gv[d];
         const uint32_t key = act ? acc_c : LOST;
-        warp_flush<NVD>(fbuf, fkey, key, acc, w.gadv, w.do_correct, cv, w.gdv);
+        if constexpr (WinFlush<NVD>::SETS == 2) {
+            warp_flush<NVD>(fbuf, fkey, key, acc, w.gadv, w.do_correct, cv, w.gdv);
+        } else {
+            warp_flush<NVD>(fbuf, fkey, key, acc, w.gadv);
+            if (w.do_correct) warp_flush<NVD>(fbuf, fkey, key, cv, w.gdv);
+        }
         if (act)
 #pragma unroll
             for (int d = 0; d < DIM; ++d) w.gxi[(size_t)d * w.n + p] = g[d];
@@ -823,16 +846,6 @@ inline int win_forward_t(const WinArgs& w, cudaStream_t s)
     return n;
 }
 
-template <int DIM, typename Real, bool AFF>
-inline void win_rev_launch(const WinArgs& w, int j, cudaStream_t s)
-{
-    constexpr int smem = 4 * 2 * (1 << DIM) * DIM * WF_ROW * (int)sizeof(double);  // 17 KB in 2D, 51 KB in 3D
-    auto* kernel = k_win_rev<DIM, Real, AFF>;
-    static const cudaError_t sized = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    (void)sized;
-    kernel<<<occupancy_grid((const void*)kernel, 128, smem), 128, smem, s>>>(w, j);
-}
-
 // Segments in reverse: replay (recording) unless the record buffer holds the
 // segment already (rec_seg), then the reverse sweep.
 template <int DIM, typename Real>
@@ -845,8 +858,10 @@ inline int win_backward_t(const WinArgs& w, double* g_v0, int rec_seg, cudaStrea
         const int k0 = j * w.C, k1 = k0 + w.C < w.K ? k0 + w.C : w.K;
         if (j != rec_seg)
             for (int k = k0; k < k1; ++k) n += win_step<DIM, Real, true>(w, k, k0, 1, s);
-        if (w.a.mesh.all_affine) win_rev_launch<DIM, Real, true>(w, j, s);
-        else win_rev_launch<DIM, Real, false>(w, j, s);
+        if (w.a.mesh.all_affine)
+            k_win_rev<DIM, Real, true><<<win_grid(k_win_rev<DIM, Real, true>, 128), 128, 0, s>>>(w, j);
+        else
+            k_win_rev<DIM, Real, false><<<win_grid(k_win_rev<DIM, Real, false>, 128), 128, 0, s>>>(w, j);
         n += 1;
     }
     return n;
