@@ -29,17 +29,33 @@ inline int occupancy_grid(const void* kernel, int threads, size_t smem = 0)
     return g;
 }
 
-// Whether the advect pass takes quarter chunks: fewer than 4 whole chunks per
-// block of the whole-chunk grid at two particles per cell part.
-inline bool small_advect(const StepArgs& a, int grid)
+// Particles a launch is sized for: near what a long run settles at, 1.9 per
+// cell part at max 2 and 4.4 at max 5, within what the arrays hold.  (Sized
+// for 2 per part whatever the max, FP64 advect at max 5 took 21 us for a
+// channel of 64x16 cells of 2x2 parts and 29 for a duct of 48x12x12 of
+// 2x2x2, so it takes 15 and 24.)
+inline long long expected_particles(const StepArgs& a)
 {
-    return 2ll * (a.cend - a.cbeg) * a.pp.npart < 4ll * grid * ADV_CH;
+    const long long n = (long long)(a.cend - a.cbeg) * a.pp.npart * (a.pp.maxpp > 2 ? a.pp.maxpp : 2);
+    return n < (long long)a.capacity ? n : (long long)a.capacity;
 }
 
-// Their grid: at most one block per quarter chunk of that many particles.
+// Whether the advect pass takes quarter chunks: up to 4 whole chunks per
+// block of the whole-chunk grid (FP32, channel 64x16 with 26 k particles: 9
+// against 12 us; duct 64x16x16 with 0.85 M: 29 against 31), but not where whole
+// chunks fill the grid once and quarters, on twice the blocks of half the
+// threads, would need a second round (duct 48x12x12 at max 5, 0.25 M: 15
+// against 17 us; cube 16^3, 0.21 M: 19 against 23).
+inline bool small_advect(const StepArgs& a, int grid)
+{
+    const long long n = expected_particles(a), round = (long long)grid * ADV_CH;
+    return n < 4 * round && !(n > round / 2 && n <= round);
+}
+
+// Their grid: at most one block per quarter chunk.
 inline int small_grid(const StepArgs& a, int grid, int chunk)
 {
-    const long long n = (2ll * (a.cend - a.cbeg) * a.pp.npart + chunk - 1) / chunk;
+    const long long n = (expected_particles(a) + chunk - 1) / chunk;
     return n < 1 ? 1 : n < grid ? (int)n : grid;
 }
 
