@@ -29,8 +29,9 @@ struct pfem2gpu_handle {
             *d2c_ent = nullptr;
     double *verts = nullptr, *cellX = nullptr, *aff = nullptr, *v2c_dirs = nullptr, *v2c_rec = nullptr;
     float* geo32 = nullptr;
-    uint32_t* twisted = nullptr;  // cells whose map is not affine; 3D cells unfit for locate_lin64 (set by cell_setup)
-    bool all_affine = false, lin64 = false;
+    // set by cell_setup: cells whose map is not affine; 3D cells unfit for locate_lin64; largest cell; ~ smallest
+    uint32_t* twisted = nullptr;
+    bool all_affine = false, lin64 = false, uneven = false;
     uint8_t* mild = nullptr;  // 2D: cells whose closed-form inverse decides (mild_quad64)
     // velocities
     double *Vstage = nullptr, *Vstage2 = nullptr, *Vout = nullptr;
@@ -217,6 +218,7 @@ StepArgs args(pfem2gpu_handle* h)
     a.mesh.nC = h->nC;
     a.mesh.all_affine = h->all_affine ? 1 : 0;
     a.mesh.lin64 = h->lin64 ? 1 : 0;
+    a.mesh.uneven = h->uneven ? 1 : 0;
     a.mesh.mild = h->mild;
     a.mesh.nV = h->nV;
     a.mesh.nD = h->nD;
@@ -1164,8 +1166,8 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
     }
     CK(dalloc(&h->jinv32, nc * (dim == 3 ? 12 : 8)));
     if (dim == 2) CK(dalloc(&h->mild, nc));
-    CK(dalloc(&h->twisted, 2));
-    CK(cudaMemsetAsync(h->twisted, 0, 8, h->stream));
+    CK(dalloc(&h->twisted, 4));
+    CK(cudaMemsetAsync(h->twisted, 0, 16, h->stream));
     CK(cudaMalloc(&h->partials, nc * PW * esize(h)));
     CK(cudaMemcpyAsync(h->cv, cell_vertices, nc * NV * 4, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->cd, cell_dofs, nc * NV * 4, cudaMemcpyHostToDevice, h->stream));
@@ -1181,11 +1183,16 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
             return launch_cell_setup(dim, h->nC, h->verts, h->cv, h->cellX, h->aff, h->geo32, h->jinv32, h->twisted,
                                      h->mild, h->stream);
         });
-    uint32_t twisted[2] = {0, 0};
-    CK(cudaMemcpyAsync(twisted, h->twisted, 8, cudaMemcpyDeviceToHost, h->stream));
+    uint32_t twisted[4] = {0, 0, 0, 0};
+    CK(cudaMemcpyAsync(twisted, h->twisted, 16, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));  // host vectors above go out of scope
     h->all_affine = twisted[0] == 0;
     h->lin64 = dim == 3 && twisted[1] == 0;
+    float largest = 0.0f, smallest = 0.0f;
+    const uint32_t sb = ~twisted[3];
+    memcpy(&largest, &twisted[2], 4);
+    memcpy(&smallest, &sb, 4);
+    h->uneven = twisted[3] != 0 && largest > 8.0f * smallest;
     h->has_mesh = true;
     h->vaos_valid = false;
     h->gen++;

@@ -64,6 +64,7 @@ struct MeshDev {
     int nC, nV, nD;
     int all_affine;           // 1 if every cell's multilinear map is affine (no twist terms)
     int lin64;                // 3D: 1 if locate_lin64 holds for every cell
+    int uneven;               // 1 if the largest cell has more than 8 times the smallest one's volume
     const uint8_t* mild;      // 2D: per cell, mild_quad64 (null: 3D)
     const int32_t* cv;        // nC x NV vertex ids
     const int32_t* cd;        // nC x NV DoF ids

@@ -67,7 +67,7 @@ __global__ void k_cell_setup(int nC, const double* __restrict__ verts, const int
                 J[d][DIM - 1] = Y[4 % NV][d] + 0.5 * Y[5 % NV][d] + 0.5 * Y[6 % NV][d] + 0.25 * Y[7 % NV][d];
             }
         }
-        invert64<DIM>(J, Ji);
+        const float size = fabsf((float)invert64<DIM>(J, Ji));
         float* jj = jinv32 + (size_t)c * JS;
 #pragma unroll
         for (int r = 0; r < DIM; ++r)
@@ -76,6 +76,14 @@ __global__ void k_cell_setup(int nC, const double* __restrict__ verts, const int
         for (int k = DIM * DIM; k < JS; ++k) jj[k] = 0.0f;
         jj[DIM * DIM] = affine ? 1.0f : 0.0f;
         if (!affine) atomicAdd(twisted, 1u);
+        {  // the largest and (complemented) the smallest cell, positive floats ordered by their bits
+            const unsigned am = __activemask(), bits = size > 0.0f && size < INFINITY ? __float_as_uint(size) : 0u;
+            const unsigned hi = __reduce_max_sync(am, bits), lo = __reduce_max_sync(am, bits ? ~bits : 0u);
+            if ((int)(threadIdx.x & 31) == __ffs(am) - 1) {
+                atomicMax(twisted + 2, hi);
+                atomicMax(twisted + 3, lo);
+            }
+        }
         if constexpr (DIM == 2) mild[c] = mild_quad64(X, aff + (size_t)c * Dims<DIM>::AFF) ? 1 : 0;
         if constexpr (DIM == 3)
             if (!(lin64_error(X, aff + (size_t)c * Dims<DIM>::AFF, affine) <= LIN64_MAX)) atomicAdd(twisted + 1, 1u);

@@ -340,13 +340,25 @@ __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;"
 // ---------------------------------------------------------------------------
 // Tiles.  TCAP entries (old slots, arrivals, new particles) fit one tile's
 // shared memory.  The kernel takes as many cells per tile as bring it near
-// TARGET particles at the layout's mean density, fewer where the tiles would
-// not fill the grid; a tile that holds more than TCAP is worked through in
-// runs of cells that fit, and a single cell beyond TCAP takes the general
-// path.  Sizes measured (write pass, us; FP32 duct of 7.0 M particles / cube
-// of 32 M): 512 entries, 7 blocks per SM 215 / 990; 640, 6 blocks 199 / 917;
-// 896, 5 blocks 202 / 868, which leaves smaller meshes too few tiles.  FP64
-// (duct / 37^3 cube): 384, 5 blocks 520 / 532; 512, 4 blocks 489 / 465.
+// TARGET particles at the layout's mean density, and then shares the cells
+// out over the waves of blocks this takes; a tile that holds more than TCAP is
+// worked through in runs of cells that fit, and a single cell beyond TCAP
+// takes the general path.  Sizes measured (write pass, us; FP32 duct of 7.0 M
+// particles / cube of 32 M): 512 entries, 7 blocks per SM 215 / 990; 640, 6
+// blocks 199 / 917; 896, 5 blocks 202 / 868, which leaves smaller meshes too
+// few tiles.  FP64 (duct / 37^3 cube): 384, 5 blocks 520 / 532; 512, 4 blocks
+// 489 / 465.
+//
+// Where cells differ little, more waves of smaller tiles only add tiles: with
+// 8 waves in place of 2 or 3 a 64x16x16 duct of 0.9 M particles takes 61 us
+// for 39 in FP32 and 83 for 71 in FP64, a 30^3 cube of 1.4 M 76 for 53 and
+// 109 for 103.  Where the largest cell has more than 8 times the smallest
+// one's volume, the small ones' arrivals make some tiles much the larger, and
+// smaller tiles even that out: Turek mesh, 1.9 M, FP32 4 waves 125 us, 6 89, 8
+// 94; FP64 8 waves 145, 13 137; seeded cylinder channel of 25 k cells FP32 1
+// wave 56, 5 44, 8 52.  So at least 6 waves there while a tile keeps 100
+// entries, and never more than `most` entries a tile.  (The ratio is 98 and
+// 72 on these meshes, 1.7 on the cube with its vertices moved by a tenth.)
 // ---------------------------------------------------------------------------
 constexpr int WT_CELLS = 24;  // cells per tile at most
 constexpr int WT_CNT = 1024;  // part counters of a run of cells
@@ -519,15 +531,17 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
     const int apply = a.apply_counts, maxpp = a.pp.maxpp, npe = a.pp.npe, occw = a.pp.occw;
     uint32_t NC;  // cells per tile
     {
-        // near TARGET particles at the mean density; in one wave of blocks, or in at least 8 (cells
-        // differ: on the Turek mesh 5 waves take 122 us, 8 take 100, 12 take 108), each wave full
+        // near TARGET particles at the mean density, in as few waves of blocks as that takes, each wave full
         const uint32_t total = (uint32_t)a.coff[nC];
         const unsigned long long by_load = total ? (unsigned long long)TARGET * nC / total : WT_CELLS;
         const uint32_t by_cnt = WT_CNT / npe;
         NC = by_load < WT_CELLS ? (uint32_t)by_load : WT_CELLS;
         NC = max(min(NC, by_cnt), 1u);
         uint32_t waves = (nC + NC * gridDim.x - 1) / (NC * gridDim.x);
-        if (waves > 1 && waves < 8) waves = 8;
+        if (a.mesh.uneven) {  // smaller cells are left by more of their particles: more and smaller tiles even that out
+            const uint32_t block = total / gridDim.x, most = HX ? TCAP / 2 : TCAP * 3 / 5;
+            waves = max(waves, max(min(6u, block / 100u), (block + most - 1) / most));
+        }
         NC = min(NC, (nC + waves * gridDim.x - 1) / (waves * gridDim.x));
         NC = NC < 1 ? 1 : NC;
     }
