@@ -114,6 +114,7 @@ struct StepArgs {
     const double* Va;     // staged nodal velocity, nD x VS (one row per DoF)
     int do_correct;
     int apply_counts;   // write kernel: 1 = count correction, 0 = keep all (re-sort only)
+    int light;          // write kernel, FP32 form: the instance for few particles per part (note_density)
     int count_step;     // write kernel: add the step's particles to particle_steps
     int reset_nan;      // write kernel: zero nan_dofs for the projection that follows
     uint32_t* key;      // cell after the move, or LOST

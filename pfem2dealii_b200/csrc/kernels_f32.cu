@@ -95,18 +95,19 @@ int launch_cross(int dim, int prec, const StepArgs& a, cudaStream_t s)
     return dim == 2 ? cross32_t<2, false>(a, s) : cross32_t<3, false>(a, s);
 }
 
-template <int DIM>
+template <int DIM, bool LIGHT>
 static int write32_t(const StepArgs& a, cudaStream_t s)
 {
     const int smem = (int)sizeof(WtTile<DIM, float>);
-    static const int grid = smem_grid32(k_write<DIM, float>, (WtCfg<DIM, float>::THREADS), smem);
-    return launch_pdl(k_write<DIM, float>, grid, (WtCfg<DIM, float>::THREADS), smem, s, a);
+    static const int grid = smem_grid32(k_write<DIM, float, LIGHT>, (WtCfg<DIM, float>::THREADS), smem);
+    return launch_pdl(k_write<DIM, float, LIGHT>, grid, (WtCfg<DIM, float>::THREADS), smem, s, a);
 }
 
 int launch_write(int dim, int prec, const StepArgs& a, cudaStream_t s)
 {
     if (prec == 0) return launch64_write(dim, a, s);
-    return dim == 2 ? write32_t<2>(a, s) : write32_t<3>(a, s);
+    if (a.light) return dim == 2 ? write32_t<2, true>(a, s) : write32_t<3, true>(a, s);
+    return dim == 2 ? write32_t<2, false>(a, s) : write32_t<3, false>(a, s);
 }
 
 int launch_partials(int dim, int prec, const StepArgs& a, const uint32_t* cs, cudaStream_t s)

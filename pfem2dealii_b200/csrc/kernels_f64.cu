@@ -172,8 +172,8 @@ template <int DIM>
 static int write_t(const StepArgs& a, cudaStream_t s)
 {
     const int smem = (int)sizeof(WtTile<DIM, double>);
-    static const int grid = smem_grid(k_write<DIM, double>, (WtCfg<DIM, double>::THREADS), smem);
-    return launch_pdl(k_write<DIM, double>, grid, (WtCfg<DIM, double>::THREADS), smem, s, a);
+    static const int grid = smem_grid(k_write<DIM, double, false>, (WtCfg<DIM, double>::THREADS), smem);
+    return launch_pdl(k_write<DIM, double, false>, grid, (WtCfg<DIM, double>::THREADS), smem, s, a);
 }
 
 int launch64_write(int dim, const StepArgs& a, cudaStream_t s)

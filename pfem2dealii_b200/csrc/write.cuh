@@ -505,7 +505,10 @@ __device__ __noinline__ void ties_in_cells(const StepArgs& a, WtTile<DIM, Real>&
     if (threadIdx.x == 0) w.ties[1] = 0;
 }
 
-template <int DIM, typename Real>
+// LIGHT: an instance for layouts of few particles per part (note_density): a run
+// in whose cells no part can be over-full, by their counts and their occupied
+// parts, takes no part counts.  The two give the same results.
+template <int DIM, typename Real, bool LIGHT>
 __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>::BLOCKS))
     k_write(const __grid_constant__ StepArgs a)
 {
@@ -626,6 +629,19 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                 const uint32_t E = h.cs[ce], EA = (E + 3u) & ~3u;
                 const uint32_t nold = h.cs[cb] < E ? EA - SA : 0u, narr = h.aoff[ce] - a0;
                 const uint32_t nE = nold + narr, nT = nE + (h.co[ce].y - sb0);
+                // LIGHT, a cell per lane: can a part be over-full (the cell's count exceeds its occupied parts by
+                // more than max)?  And the cells whose sums go by the old slots' rows (see there).
+                bool count = true;
+                uint32_t rows = 0;
+                if constexpr (LIGHT) {
+                    const uint32_t lc = cb + lane < ce ? cb + lane : cb;
+                    const uint32_t nseed = h.co[lc + 1].y - h.co[lc].y, n = h.co[lc + 1].x - h.co[lc].x - nseed;
+                    uint32_t occ = 0;
+                    for (int q = 0; q < occw; ++q) occ += __popcll(h.occ[lc * occw + q]);
+                    const bool over = apply && !(maxpp >= 0 && n <= occ + (uint32_t)maxpp);
+                    rows = __ballot_sync(0xffffffffu, nseed == 0 && h.cs[lc + 1] - h.cs[lc] + h.na[lc] <= 32u && !over);
+                    count = __any_sync(0xffffffffu, over);
+                }
                 if (nold) {
                     if (stage_ok) {
                         if (tid == 0) {
@@ -698,7 +714,8 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                         w.meta[e] = (uint16_t)NONE;
                     }
                 }
-                for (uint32_t t = tid; t < (ce - cb) * npe; t += THREADS) w.cnt[t] = 0;
+                if (!LIGHT || count)
+                    for (uint32_t t = tid; t < (ce - cb) * npe; t += THREADS) w.cnt[t] = 0;
                 // new particles, while the copies are in flight: the real parts the move left empty
                 {
                     uint32_t todo = __ballot_sync(0xffffffffu, cb + lane < ce && h.co[cb + lane + 1].y != h.co[cb + lane].y);
@@ -753,9 +770,7 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                 // cell and part of every entry; part counts.  Entry r * THREADS + tid stays in this thread's
                 // registers; word r * WARPS + warp of the survivors is this warp's.
                 uint32_t m[ROUNDS];
-#pragma unroll
-                for (int r = 0; r < ROUNDS; ++r) {
-                    const uint32_t e = r * THREADS + tid;
+                auto place = [&](int r, uint32_t e) {
                     m[r] = NONE;
                     if (e < nold) {
                         const uint32_t lc = w.key[e] - c0, slot = SA + e;
@@ -764,54 +779,70 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                         m[r] = w.meta[e];
                         if (e < nE) w.key[e] = m[r] != NONE ? key_of(w.id[e], a.pp.seed) : ~0u;
                     }
-                    if (e < nE && m[r] != NONE) {
-                        Real xi[DIM];
+                };
+                if (!LIGHT || count) {
 #pragma unroll
-                        for (int d = 0; d < DIM; ++d) xi[d] = w.xi[d][e];
-                        const int pe = ext_part<DIM, Real>(xi, a.pp);
-                        if (apply) atomicAdd(w.cnt + ((m[r] >> 8) - cb) * npe + pe, 1);
-                        m[r] |= (uint32_t)pe;
-                    }
-                }
-                __syncthreads();
-                // survivors: everyone outside the over-full parts, and there the smallest keys
-                bool over = false;
+                    for (int r = 0; r < ROUNDS; ++r) {
+                        const uint32_t e = r * THREADS + tid;
+                        place(r, e);
+                        if (e < nE && m[r] != NONE) {
+                            Real xi[DIM];
 #pragma unroll
-                for (int r = 0; r < ROUNDS; ++r) {
-                    const uint32_t e = r * THREADS + tid;
-                    bool live = e < nE && m[r] != NONE;
-                    if (live && apply && w.cnt[((m[r] >> 8) - cb) * npe + (m[r] & 255u)] > maxpp + 1) {
-                        w.perm[atomicAdd(&w.nover, 1u)] = (uint16_t)e;
-                        w.meta[e] = (uint16_t)m[r];
-                        over = true;
-                        live = false;
-                    }
-                    const unsigned b = __ballot_sync(0xffffffffu, live);
-                    if (lane == 0) w.mask[r * WARPS + warp] = b;
-                }
-                if (__syncthreads_or(over)) {
-                    const uint32_t nov = w.nover;
-                    int tie = 0;
-                    for (uint32_t j = tid; j < nov; j += THREADS) {
-                        const uint32_t e = w.perm[j], me = w.meta[e], kk = key_of(w.id[e], a.pp.seed);
-                        int rank = 0;
-                        for (uint32_t o = 0; o < nov; ++o) {
-                            const uint32_t f = w.perm[o], kf = key_of(w.id[f], a.pp.seed);
-                            rank += (w.meta[f] == me && kf < kk) ? 1 : 0;
-                        }
-                        tie += 2 * rank - (w.cnt[((me >> 8) - cb) * npe + (me & 255u)] - 1);
-                        if (rank < maxpp + 1) {
-                            atomicOr(w.mask + (e >> 5), 1u << (e & 31u));
-                        } else {
-                            w.key[e] = ~0u;
-                            removed++;
+                            for (int d = 0; d < DIM; ++d) xi[d] = w.xi[d][e];
+                            const int pe = ext_part<DIM, Real>(xi, a.pp);
+                            if (apply) atomicAdd(w.cnt + ((m[r] >> 8) - cb) * npe + pe, 1);
+                            m[r] |= (uint32_t)pe;
                         }
                     }
-                    tie = __reduce_add_sync(0xffffffffu, tie);
-                    if (lane == 0 && tie) atomicAdd(&w.ties[0], tie);
                     __syncthreads();
-                    if (w.ties[0]) removed += ties_in_parts<DIM, Real>(a, w, hb, c0, cb, ce, nov);
-                    if (tid == 0) w.nover = 0;
+                    // survivors: everyone outside the over-full parts, and there the smallest keys
+                    bool over = false;
+#pragma unroll
+                    for (int r = 0; r < ROUNDS; ++r) {
+                        const uint32_t e = r * THREADS + tid;
+                        bool live = e < nE && m[r] != NONE;
+                        if (live && apply && w.cnt[((m[r] >> 8) - cb) * npe + (m[r] & 255u)] > maxpp + 1) {
+                            w.perm[atomicAdd(&w.nover, 1u)] = (uint16_t)e;
+                            w.meta[e] = (uint16_t)m[r];
+                            over = true;
+                            live = false;
+                        }
+                        const unsigned b = __ballot_sync(0xffffffffu, live);
+                        if (lane == 0) w.mask[r * WARPS + warp] = b;
+                    }
+                    if (__syncthreads_or(over)) {
+                        const uint32_t nov = w.nover;
+                        int tie = 0;
+                        for (uint32_t j = tid; j < nov; j += THREADS) {
+                            const uint32_t e = w.perm[j], me = w.meta[e], kk = key_of(w.id[e], a.pp.seed);
+                            int rank = 0;
+                            for (uint32_t o = 0; o < nov; ++o) {
+                                const uint32_t f = w.perm[o], kf = key_of(w.id[f], a.pp.seed);
+                                rank += (w.meta[f] == me && kf < kk) ? 1 : 0;
+                            }
+                            tie += 2 * rank - (w.cnt[((me >> 8) - cb) * npe + (me & 255u)] - 1);
+                            if (rank < maxpp + 1) {
+                                atomicOr(w.mask + (e >> 5), 1u << (e & 31u));
+                            } else {
+                                w.key[e] = ~0u;
+                                removed++;
+                            }
+                        }
+                        tie = __reduce_add_sync(0xffffffffu, tie);
+                        if (lane == 0 && tie) atomicAdd(&w.ties[0], tie);
+                        __syncthreads();
+                        if (w.ties[0]) removed += ties_in_parts<DIM, Real>(a, w, hb, c0, cb, ce, nov);
+                        if (tid == 0) w.nover = 0;
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < ROUNDS; ++r) {
+                        const uint32_t e = r * THREADS + tid;
+                        place(r, e);
+                        const unsigned b = __ballot_sync(0xffffffffu, e < nE && m[r] != NONE);
+                        if (lane == 0) w.mask[r * WARPS + warp] = b;
+                    }
+                    __syncthreads();
                 }
                 // survivors before an entry: words by a scan over the lanes, bits by a count
                 const uint32_t word = lane < TCAP / 32 ? w.mask[lane] : 0u;
@@ -920,8 +951,8 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                         // no new particles, none removed by its counts alone (the cell's count exceeds its
                         // occupied parts by at most max) and one round: rows are the old slots, then the
                         // arrivals, with the leavers' rows empty
-                        bool simple = nseed == 0 && L + na <= 32u;
-                        if (simple && apply) {
+                        bool simple = LIGHT ? ((rows >> (lc - cb)) & 1u) != 0u : nseed == 0 && L + na <= 32u;
+                        if (!LIGHT && simple && apply) {
                             uint32_t occ = 0;
                             for (int q = 0; q < occw; ++q) occ += __popcll(h.occ[lc * occw + q]);
                             simple = maxpp >= 0 && ub <= occ + (uint32_t)maxpp;
