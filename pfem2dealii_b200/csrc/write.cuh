@@ -97,113 +97,6 @@ __device__ __forceinline__ uint2 write_seeds(const StepArgs& a, uint32_t c, cons
     return make_uint2(done, err);
 }
 
-// One cell of any particle count (one warp), for the cells that fit no tile.
-// Per-element data goes to the cell's own slot range of the scratch array;
-// survivors and positions are found by counting.  Order: stayers by slot,
-// arrivals by key, new particles by part -- the same as the tiles'.
-template <int DIM, typename Real>
-__device__ __noinline__ uint2 write_cell_general(const StepArgs& a, int* cnt, Real (*tr)[TRW], uint32_t c, uint32_t s0,
-                                                 uint32_t L, uint32_t na, uint32_t h, uint32_t off, uint32_t ub,
-                                                 uint32_t nseed_expect, uint32_t sb, uint32_t id0, int lane)
-{
-    uint32_t removed = 0, err = 0;
-    uint4* G = a.gscr + off;  // element -> (particle index, part, key, flags: 1 stayer, 2 survivor)
-    const int npe = a.pp.npe;
-    for (int p = lane; p < npe; p += 32) cnt[p] = 0;
-    __syncwarp();
-    if (off + ub > a.capacity) return make_uint2(0u, ERR_CAPACITY);
-    // stayers: elements 0..ns-1 in slot order
-    uint32_t ns = 0;
-    for (uint32_t base = 0; base < L; base += 32) {
-        const uint32_t j = base + lane;
-        const bool stay = j < L && a.key[s0 + j] == c;
-        const unsigned m = __ballot_sync(0xffffffffu, stay);
-        if (stay) {
-            const uint32_t i = s0 + j, e = ns + __popc(m & ((1u << lane) - 1u));
-            Real xi[DIM];
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) xi[d] = ldr<Real>(a.T.xi[d], i);
-            const int pe = ext_part<DIM, Real>(xi, a.pp);
-            if (e < ub) G[e] = make_uint4(i, (uint32_t)pe, key_of(a.S0.id[i], a.pp.seed), 1u);
-            atomicAdd(cnt + pe, 1);
-        }
-        ns += __popc(m);
-    }
-    // arrivals: elements ns.. (slots lane-parallel; the overflow list walked by all lanes)
-    uint32_t t = 0, p = h;
-    for (; t < na && t < a.capacity; ++t) {
-        uint32_t i;
-        if (t < (uint32_t)ARRCAP) {
-            i = a.carrs[(size_t)c * ARRCAP + t];
-        } else {
-            if (p == LOST) break;
-            i = p;
-            p = a.next[p];
-        }
-        if ((t & 31u) == (uint32_t)lane) {
-            Real xi[DIM];
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) xi[d] = ldr<Real>(a.T.xi[d], i);
-            const int pe = ext_part<DIM, Real>(xi, a.pp);
-            if (ns + t < ub) G[ns + t] = make_uint4(i, (uint32_t)pe, key_of(a.S0.id[i], a.pp.seed), 0u);
-            atomicAdd(cnt + pe, 1);
-        }
-    }
-    const uint32_t n = ns + t;
-    __syncwarp();
-    __threadfence_block();
-    if (n > ub) return make_uint2(0u, ERR_COUNT_UB);
-    // survivors: rank by key inside the part
-    uint32_t nsurv = 0;
-    for (uint32_t e = lane; e < n; e += 32) {
-        const uint4 g = G[e];
-        const int k = cnt[g.y];
-        int rank = 0;
-        if (a.apply_counts && k > a.pp.maxpp + 1)
-            for (uint32_t m = 0; m < n; ++m) {
-                const uint4 o = G[m];
-                rank += (o.y == g.y && (o.z < g.z || (o.z == g.z && o.x < g.x))) ? 1 : 0;
-            }
-        if (rank < survivors(k, a.pp.maxpp, a.apply_counts)) {
-            G[e].w = g.w | 2u;
-            nsurv++;
-        } else {
-            removed++;
-        }
-    }
-    nsurv = __reduce_add_sync(0xffffffffu, nsurv);
-    __syncwarp();
-    __threadfence_block();
-    // positions: survivors before in (stayers by slot | arrivals by key) order
-    for (uint32_t e = lane; e < n; e += 32) {
-        const uint4 g = G[e];
-        if (!(g.w & 2u)) continue;
-        const bool gs = g.w & 1u;
-        uint32_t pos = 0;
-        for (uint32_t m = 0; m < n; ++m) {
-            const uint4 o = G[m];
-            if (!(o.w & 2u)) continue;
-            const bool os = o.w & 1u;
-            const bool less = os ? o.x < g.x : o.z < g.z || (o.z == g.z && o.x < g.x);
-            pos += ((os && !gs) || (os == gs && less)) ? 1u : 0u;
-        }
-        PData<DIM, Real> pd;
-        load_global<DIM, Real>(a, g.x, pd);
-        store_particle<DIM, Real>(a, off + pos, c, pd);
-    }
-    const uint2 sd = write_seeds<DIM, Real>(a, c, cnt, n, off + nsurv, id0, sb, lane);
-    err |= sd.y;
-    const uint32_t nseed = sd.x;
-    const uint32_t fin = nsurv + nseed;
-    if (nseed != nseed_expect) err |= ERR_COUNT;
-    if (fin > ub) err |= ERR_COUNT_UB;
-    write_holes(a, off + fin, off + ub, lane);
-    __syncwarp();
-    __threadfence_block();
-    partials_of_range<DIM, Real>(a, a.S1, c, off, fin < ub ? fin : ub, tr, lane);
-    return make_uint2(removed, err);
-}
-
 // A cell's new range [off, off + ub), within the capacity, and the advect
 // chunks' recorded slots (ADV_REC) in it.
 __device__ __forceinline__ void new_range(const StepArgs& a, uint32_t c, uint32_t off, uint32_t ub)
@@ -372,6 +265,133 @@ struct WtCfg {
     static constexpr int TARGET = HX ? 470 : 600;
     static constexpr int WARPS = 4, THREADS = WARPS * 32, BLOCKS = HX ? 4 : 6;
 };
+
+// One cell of any particle count (the whole block), for the cells that fit no
+// tile.  Per-element data goes to the cell's own slot range of the scratch
+// array; survivors and positions are found by counting.  Order: stayers by
+// slot, arrivals by key, new particles by part -- the same as the tiles'.
+// Quadratic in the cell's particles, so all threads share the counting: with
+// one warp of the block at it a 64x16x16 duct of 54 a cell with 800 in one of
+// 50 took 6354 us in FP32 and 8679 in FP64 (a warp per cell before the tiles
+// 4164 and 3779), now 1716 and 2262; 1536 cells of 700 3950 and 5408, now 1274
+// and 1733.
+template <int DIM, typename Real>
+__device__ __noinline__ uint2 write_cell_general(const StepArgs& a, int* cnt, uint32_t* sc, Real (*tr)[TRW], uint32_t c,
+                                                 uint32_t s0, uint32_t L, uint32_t na, uint32_t h, uint32_t off,
+                                                 uint32_t ub, uint32_t nseed_expect, uint32_t sb, uint32_t id0)
+{
+    constexpr int WARPS = WtCfg<DIM, Real>::WARPS, THREADS = WtCfg<DIM, Real>::THREADS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint32_t removed = 0, err = 0;
+    uint4* G = a.gscr + off;  // element -> (particle index, part, key, flags: 1 stayer, 2 survivor)
+    const int npe = a.pp.npe;
+    for (int p = tid; p < npe; p += THREADS) cnt[p] = 0;
+    if (tid == 0) sc[WARPS] = 0;  // survivors
+    __syncthreads();
+    if (off + ub > a.capacity) return make_uint2(0u, ERR_CAPACITY);
+    // stayers: elements 0..ns-1 in slot order
+    uint32_t ns = 0;
+    for (uint32_t base = 0; base < L; base += THREADS) {
+        const uint32_t j = base + tid;
+        const bool stay = j < L && a.key[s0 + j] == c;
+        const unsigned m = __ballot_sync(0xffffffffu, stay);
+        if (lane == 0) sc[warp] = __popc(m);
+        __syncthreads();
+        uint32_t before = ns;
+#pragma unroll
+        for (int k = 0; k < WARPS; ++k) {
+            before += k < warp ? sc[k] : 0u;
+            ns += sc[k];
+        }
+        if (stay) {
+            const uint32_t i = s0 + j, e = before + __popc(m & ((1u << lane) - 1u));
+            Real xi[DIM];
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) xi[d] = ldr<Real>(a.T.xi[d], i);
+            const int pe = ext_part<DIM, Real>(xi, a.pp);
+            if (e < ub) G[e] = make_uint4(i, (uint32_t)pe, key_of(a.S0.id[i], a.pp.seed), 1u);
+            atomicAdd(cnt + pe, 1);
+        }
+        __syncthreads();
+    }
+    // arrivals: elements ns.. (slots in parallel; the overflow list walked by all threads)
+    uint32_t t = 0, p = h;
+    for (; t < na && t < a.capacity; ++t) {
+        uint32_t i;
+        if (t < (uint32_t)ARRCAP) {
+            i = a.carrs[(size_t)c * ARRCAP + t];
+        } else {
+            if (p == LOST) break;
+            i = p;
+            p = a.next[p];
+        }
+        if (t % THREADS == (uint32_t)tid) {
+            Real xi[DIM];
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) xi[d] = ldr<Real>(a.T.xi[d], i);
+            const int pe = ext_part<DIM, Real>(xi, a.pp);
+            if (ns + t < ub) G[ns + t] = make_uint4(i, (uint32_t)pe, key_of(a.S0.id[i], a.pp.seed), 0u);
+            atomicAdd(cnt + pe, 1);
+        }
+    }
+    const uint32_t n = ns + t;
+    __syncthreads();
+    if (n > ub) return make_uint2(0u, ERR_COUNT_UB);
+    // survivors: rank by key (equal ones by particle) inside the part
+    uint32_t nsurv = 0;
+    for (uint32_t e = tid; e < n; e += THREADS) {
+        const uint4 g = G[e];
+        const int k = cnt[g.y];
+        int rank = 0;
+        if (a.apply_counts && k > a.pp.maxpp + 1) {
+#pragma unroll 8
+            for (uint32_t m = 0; m < n; ++m) {
+                const uint4 o = G[m];
+                rank += (o.y == g.y && (o.z < g.z || (o.z == g.z && o.x < g.x))) ? 1 : 0;
+            }
+        }
+        if (rank < survivors(k, a.pp.maxpp, a.apply_counts)) {
+            G[e].w = g.w | 2u;
+            nsurv++;
+        } else {
+            removed++;
+        }
+    }
+    nsurv = __reduce_add_sync(0xffffffffu, nsurv);
+    if (lane == 0) atomicAdd(&sc[WARPS], nsurv);
+    __syncthreads();
+    nsurv = sc[WARPS];
+    // positions: survivors before in (stayers by slot | arrivals by key) order
+    for (uint32_t e = tid; e < n; e += THREADS) {
+        const uint4 g = G[e];
+        if (!(g.w & 2u)) continue;
+        const bool gs = g.w & 1u;
+        uint32_t pos = 0;
+#pragma unroll 8
+        for (uint32_t m = 0; m < n; ++m) {
+            const uint4 o = G[m];
+            const bool os = o.w & 1u;
+            const bool less = os ? o.x < g.x : o.z < g.z || (o.z == g.z && o.x < g.x);
+            pos += ((o.w & 2u) && ((os && !gs) || (os == gs && less))) ? 1u : 0u;
+        }
+        PData<DIM, Real> pd;
+        load_global<DIM, Real>(a, g.x, pd);
+        store_particle<DIM, Real>(a, off + pos, c, pd);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const uint2 sd = write_seeds<DIM, Real>(a, c, cnt, n, off + nsurv, id0, sb, lane);
+        err |= sd.y;
+        const uint32_t fin = nsurv + sd.x;
+        if (sd.x != nseed_expect) err |= ERR_COUNT;
+        if (fin > ub) err |= ERR_COUNT_UB;
+        write_holes(a, off + fin, off + ub, lane);
+        __syncwarp();
+        __threadfence_block();
+        partials_of_range<DIM, Real>(a, a.S1, c, off, fin < ub ? fin : ub, tr, lane);
+    }
+    return make_uint2(removed, err);
+}
 
 // What a tile needs to know of its cells, copied while the tile before it is
 // worked on.
@@ -613,16 +633,13 @@ __global__ void __launch_bounds__((WtCfg<DIM, Real>::THREADS), (WtCfg<DIM, Real>
                 ce = cb + (uint32_t)__popc(__ballot_sync(0xffffffffu, fits));
             }
             if (ce == cb) {  // a single cell beyond a tile
-                if (warp == 0) {
-                    const uint32_t c = c0 + cb, ub = h.co[cb + 1].x - ob;
-                    auto* tr = reinterpret_cast<Real(*)[TRW]>(&w.xi[0][0]);  // rows where a tile's entries would be
-                    const uint2 gr =
-                        write_cell_general<DIM, Real>(a, w.cnt, tr, c, h.cs[cb], h.cs[cb + 1] - h.cs[cb], h.na[cb],
-                                                      a.head[c], ob, ub, h.co[cb + 1].y - sb0, sb0, id0, lane);
-                    if (lane == 0) new_range(a, c, ob, ub);
-                    removed += gr.x;
-                    err |= gr.y;
-                }
+                const uint32_t c = c0 + cb, ub = h.co[cb + 1].x - ob;
+                auto* tr = reinterpret_cast<Real(*)[TRW]>(&w.xi[0][0]);  // rows where a tile's entries would be
+                const uint2 gr = write_cell_general<DIM, Real>(a, w.cnt, w.mask, tr, c, h.cs[cb], h.cs[cb + 1] - h.cs[cb],
+                                                               h.na[cb], a.head[c], ob, ub, h.co[cb + 1].y - sb0, sb0, id0);
+                if (tid == 0) new_range(a, c, ob, ub);
+                removed += gr.x;
+                err |= gr.y;
                 ce = cb + 1;
             } else {
                 // Entries: the old slots [SA, EA), the arrivals, the new particles.
