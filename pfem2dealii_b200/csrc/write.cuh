@@ -288,7 +288,12 @@ __device__ __noinline__ uint2 write_cell_general(const StepArgs& a, int* cnt, ui
     for (int p = tid; p < npe; p += THREADS) cnt[p] = 0;
     if (tid == 0) sc[WARPS] = 0;  // survivors
     __syncthreads();
-    if (off + ub > a.capacity) return make_uint2(0u, ERR_CAPACITY);
+    // nothing is written for a cell that does not fit: its slots are empty, not what stood there two steps ago
+    auto refuse = [&](uint32_t flag) {
+        for (uint32_t j = off + tid; j < off + ub && j < a.capacity; j += THREADS) a.S1.cell[j] = HOLE;
+        return make_uint2(0u, flag);
+    };
+    if (off + ub > a.capacity) return refuse(ERR_CAPACITY);
     // stayers: elements 0..ns-1 in slot order
     uint32_t ns = 0;
     for (uint32_t base = 0; base < L; base += THREADS) {
@@ -336,7 +341,7 @@ __device__ __noinline__ uint2 write_cell_general(const StepArgs& a, int* cnt, ui
     }
     const uint32_t n = ns + t;
     __syncthreads();
-    if (n > ub) return make_uint2(0u, ERR_COUNT_UB);
+    if (n > ub) return refuse(ERR_COUNT_UB);
     // survivors: rank by key (equal ones by particle) inside the part
     uint32_t nsurv = 0;
     for (uint32_t e = tid; e < n; e += THREADS) {
