@@ -35,30 +35,19 @@ int launch_seed(int dim, int prec, const StepArgs& a, uint32_t* cs, cudaStream_t
     return 1;
 }
 
-template <typename K>
-static int smem_grid32(K kernel, int threads, int smem)
-{
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
-    return sms * (per > 0 ? per : 1);
-}
-
 // RK: the midpoint sub-step (params.integrator = PFEM2GPU_RK2), compiled as
 // its own kernels so that the Euler ones carry no trace of it.
 template <int DIM, bool RK, bool AFF>
 static int advect32_a(const StepArgs& a, cudaStream_t s)
 {
     const auto smem = [](int stage) { return 2 * (stage + (int)sizeof(AdvRecStage<DIM>)); };
-    static const int grid = smem_grid32(k_advect32<DIM, AFF, RK, ADV_CH>, adv_threads(ADV_CH),
-                                        smem(sizeof(AdvStage<DIM, float, ADV_CH>)));
+    const int grid = smem_grid(k_advect32<DIM, AFF, RK, ADV_CH>, adv_threads(ADV_CH),
+                               smem(sizeof(AdvStage<DIM, float, ADV_CH>)));
     if (!small_advect(a, grid))
         return launch_pdl(k_advect32<DIM, AFF, RK, ADV_CH>, grid, adv_threads(ADV_CH),
                           smem(sizeof(AdvStage<DIM, float, ADV_CH>)), s, a);
-    static const int grid_s = smem_grid32(k_advect32<DIM, AFF, RK, ADV_SMALL_CH>, adv_threads(ADV_SMALL_CH),
-                                          smem(sizeof(AdvStage<DIM, float, ADV_SMALL_CH>)));
+    const int grid_s = smem_grid(k_advect32<DIM, AFF, RK, ADV_SMALL_CH>, adv_threads(ADV_SMALL_CH),
+                                 smem(sizeof(AdvStage<DIM, float, ADV_SMALL_CH>)));
     return launch_pdl(k_advect32<DIM, AFF, RK, ADV_SMALL_CH>, small_grid(a, grid_s, ADV_SMALL_CH), adv_threads(ADV_SMALL_CH),
                       smem(sizeof(AdvStage<DIM, float, ADV_SMALL_CH>)), s, a);
 }
@@ -99,7 +88,7 @@ template <int DIM, bool LIGHT>
 static int write32_t(const StepArgs& a, cudaStream_t s)
 {
     const int smem = (int)sizeof(WtTile<DIM, float>);
-    static const int grid = smem_grid32(k_write<DIM, float, LIGHT>, (WtCfg<DIM, float>::THREADS), smem);
+    const int grid = smem_grid(k_write<DIM, float, LIGHT>, (WtCfg<DIM, float>::THREADS), smem);
     return launch_pdl(k_write<DIM, float, LIGHT>, grid, (WtCfg<DIM, float>::THREADS), smem, s, a);
 }
 

@@ -118,24 +118,13 @@ int launch64_seed(int dim, const StepArgs& a, uint32_t* cs, cudaStream_t s)
 
 #define PFEM2_GRID(kern, thr) occupancy_grid((const void*)(kern), (thr))
 
-template <typename K>
-static int smem_grid(K kernel, int threads, int smem)
-{
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
-    return sms * (per > 0 ? per : 1);
-}
-
 // RK: the midpoint sub-step (params.integrator = PFEM2GPU_RK2), compiled as
 // its own kernels so that the Euler ones carry no trace of it.
 template <int DIM, bool RK, bool LIN>
 static int advect_l(const StepArgs& a, cudaStream_t s)
 {
     constexpr int smem = 2 * (int)(sizeof(AdvStage<DIM, double, ADV_SMALL_CH>) + (LIN ? sizeof(AdvLin64Stage) : 0));
-    static const int grid = smem_grid(k_advect64<DIM, RK, LIN>, adv_threads(ADV_SMALL_CH), smem);
+    const int grid = smem_grid(k_advect64<DIM, RK, LIN>, adv_threads(ADV_SMALL_CH), smem);
     return launch_pdl(k_advect64<DIM, RK, LIN>, small_grid(a, grid, ADV_SMALL_CH), adv_threads(ADV_SMALL_CH), smem, s, a);
 }
 
@@ -172,7 +161,7 @@ template <int DIM>
 static int write_t(const StepArgs& a, cudaStream_t s)
 {
     const int smem = (int)sizeof(WtTile<DIM, double>);
-    static const int grid = smem_grid(k_write<DIM, double, false>, (WtCfg<DIM, double>::THREADS), smem);
+    const int grid = smem_grid(k_write<DIM, double, false>, (WtCfg<DIM, double>::THREADS), smem);
     return launch_pdl(k_write<DIM, double, false>, grid, (WtCfg<DIM, double>::THREADS), smem, s, a);
 }
 

@@ -29,6 +29,26 @@ inline int occupancy_grid(const void* kernel, int threads, size_t smem = 0)
     return g;
 }
 
+// The same for kernels whose dynamic shared memory may need its limit raised,
+// which is a setting of the kernel on one device: once per device.
+template <typename K>
+inline int smem_grid(K kernel, int threads, int smem)
+{
+    static std::mutex mu;
+    static std::unordered_map<const void*, int> cache[16];  // per device
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    auto& on_dev = cache[dev & 15];
+    auto it = on_dev.find((const void*)kernel);
+    if (it != on_dev.end()) return it->second;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    int sms = 0, per = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
+    return on_dev[(const void*)kernel] = sms * (per > 0 ? per : 1);
+}
+
 // Particles a launch is sized for: near what a long run settles at, 1.9 per
 // cell part at max 2 and 4.4 at max 5, within what the arrays hold.  (Sized
 // for 2 per part whatever the max, FP64 advect at max 5 took 21 us for a
