@@ -964,7 +964,7 @@ int pfem2gpu_create(int dim, int precision, const pfem2gpu_params* prm, pfem2gpu
     }
     pp.npart = npart;
     pp.npe = npe;
-    pp.maxpp = prm->max_particles_per_cell_part;
+    pp.maxpp = std::min(prm->max_particles_per_cell_part, 0x3fffffff);  // the kernels add 1; no part holds more
     pp.S = prm->particle_integration_steps == 0 ? 1 : prm->particle_integration_steps;  // :34-36
     pp.dtp = prm->time_step / (double)pp.S;                                               // :38
     pp.seed = prm->removal_seed;
