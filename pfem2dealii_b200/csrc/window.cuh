@@ -509,14 +509,14 @@ __device__ __forceinline__ void warp_flush(double* buf, uint32_t* keys, uint32_t
 #pragma unroll
         for (int m = 0; m < NVD; ++m) buf[(NVD + m) * WF_ROW + lane] = vals2[m];
     __syncwarp();
-    if (lane < (two ? 2 * NVD : NVD)) {
-        double* dst = lane < NVD ? acc + lane : acc2 + (lane - NVD);
+    for (int m = lane; m < (two ? 2 * NVD : NVD); m += 32) {
+        double* dst = m < NVD ? acc + m : acc2 + (m - NVD);
         uint32_t cur = LOST;
         double s = 0.0;
 #pragma unroll 8
         for (int l = 0; l < 32; ++l) {
             const uint32_t k = keys[l];
-            const double v = buf[lane * WF_ROW + l];
+            const double v = buf[m * WF_ROW + l];
             if (k != cur) {
                 if (cur != LOST) atomicAdd(dst + (size_t)cur * NVD, s);
                 cur = k;
@@ -660,27 +660,32 @@ __global__ void __launch_bounds__(128, (WinRev<DIM, Real, AFF>::BLOCKS)) k_win_r
             }
         }
         // The recorded states stream from HBM and come PF sub-steps ahead, where there is room for them.
-        constexpr int PF = WinRev<DIM, Real, AFF>::PF, NEXT = PF > 0 ? PF - 1 : 0;
-        uint32_t pc[NEXT + 1];
-        Real px[NEXT + 1][DIM];
-        auto state = [&](int t, int q) {
-            const size_t o = (size_t)t * w.n + p;
-            pc[q] = w.rec_cell[o];
+        constexpr int PF = WinRev<DIM, Real, AFF>::PF, LAST = PF > 0 ? PF - 1 : 0;
+        uint32_t pc[LAST + 1];
+        Real px[LAST + 1][DIM];
 #pragma unroll
-            for (int d = 0; d < DIM; ++d) px[q][d] = ldw<Real>(w.rec_xi[d], o);
-        };
+        for (int q = 0; q < PF; ++q) {
+            const int t = tseg - 1 - q;
+            pc[q] = LOST;
+            if (act && t >= 0) {
+                pc[q] = w.rec_cell[(size_t)t * w.n + p];
 #pragma unroll
-        for (int q = 0; q < PF; ++q)
-            if (act && tseg - 1 - q >= 0) state(tseg - 1 - q, q);
+                for (int d = 0; d < DIM; ++d) px[q][d] = ldw<Real>(w.rec_xi[d], (size_t)t * w.n + p);
+            }
+        }
         for (int t = tseg - 1; t >= 0; --t) {
             if (!act) continue;
-            if (PF == 0) state(t, 0);
+            if constexpr (PF == 0) {
+                pc[0] = w.rec_cell[(size_t)t * w.n + p];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) px[0][d] = ldw<Real>(w.rec_xi[d], (size_t)t * w.n + p);
+            }
             const uint32_t ca = pc[0];
             double xa[DIM], y[DIM];
 #pragma unroll
             for (int d = 0; d < DIM; ++d) xa[d] = (double)px[0][d];
 #pragma unroll
-            for (int q = 0; q < NEXT; ++q) {
+            for (int q = 0; q < LAST; ++q) {
                 pc[q] = pc[q + 1];
 #pragma unroll
                 for (int d = 0; d < DIM; ++d) px[q][d] = px[q + 1][d];
@@ -689,7 +694,12 @@ __global__ void __launch_bounds__(128, (WinRev<DIM, Real, AFF>::BLOCKS)) k_win_r
                 prefetch_l1(w.Wcell + (size_t)pc[0] * NV * VS);
                 if constexpr (!AFF) prefetch_l1(m.cellX + (size_t)pc[0] * NV * DIM);
             }
-            if (PF > 0 && t >= PF) state(t - PF, NEXT);
+            if (PF > 0 && t >= PF) {
+                const size_t o = (size_t)(t - PF) * w.n + p;
+                pc[LAST] = w.rec_cell[o];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) px[LAST][d] = ldw<Real>(w.rec_xi[d], o);
+            }
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {  // y = J^-T g
                 double sy = 0.0;
