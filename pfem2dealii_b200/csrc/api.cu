@@ -25,9 +25,9 @@ struct pfem2gpu_handle {
     // mesh
     int nC = 0, nV = 0, nD = 0;
     bool has_mesh = false;
-    int32_t *cv = nullptr, *cd = nullptr, *v2c_off = nullptr, *v2c_cells = nullptr, *d2c_off = nullptr,
+    int32_t *cv = nullptr, *cd = nullptr, *v2c_off = nullptr, *d2c_off = nullptr,
             *d2c_ent = nullptr;
-    double *verts = nullptr, *cellX = nullptr, *aff = nullptr, *v2c_dirs = nullptr, *v2c_rec = nullptr;
+    double *verts = nullptr, *cellX = nullptr, *aff = nullptr, *v2c_rec = nullptr;
     float* geo32 = nullptr;
     // set by cell_setup: cells whose map is not affine; 3D cells unfit for locate_lin64; largest cell; ~ smallest
     uint32_t* twisted = nullptr;
@@ -998,8 +998,8 @@ int pfem2gpu_destroy(pfem2gpu_handle* h)
 {
     if (!h) return PFEM2GPU_ERR_ARG;
     if (h->stream) cudaStreamSynchronize(h->stream);
-    for (void* p : {(void*)h->cv, (void*)h->cd, (void*)h->v2c_off, (void*)h->v2c_cells, (void*)h->d2c_off,
-                    (void*)h->d2c_ent, (void*)h->verts, (void*)h->cellX, (void*)h->aff, (void*)h->v2c_dirs,
+    for (void* p : {(void*)h->cv, (void*)h->cd, (void*)h->v2c_off, (void*)h->d2c_off,
+                    (void*)h->d2c_ent, (void*)h->verts, (void*)h->cellX, (void*)h->aff,
                     (void*)h->geo32, (void*)h->v2c_rec, (void*)h->Va, (void*)h->Vstage, (void*)h->Vstage2, (void*)h->Vout, (void*)h->Vin, h->Vc, h->dVc,
                     (void*)h->key, (void*)h->next, (void*)h->xtmp, (void*)h->head, (void*)h->cs0, (void*)h->cs1,
                     (void*)h->carr, (void*)h->carrs, (void*)h->ccount, (void*)h->cocc, (void*)h->cub, (void*)h->coff,
@@ -1045,8 +1045,12 @@ static cudaError_t build_maps(pfem2gpu_handle* h, size_t nc, size_t nvx, size_t 
     const int dim = h->dim, NV = 1 << dim;
     const size_t nmax = std::max(nvx, nd), ntiles = (nmax + WIN_TILE - 1) / WIN_TILE + 1;
     uint32_t *cnt = nullptr, *fill = nullptr, *tsum = nullptr;
+    int32_t* cells = nullptr;  // the vertex map's two arrays, until they are packed into v2c_rec
+    double* dirs = nullptr;
     cudaError_t e = cudaSuccess;
     auto done = [&](cudaError_t r) {
+        dfree(cells);
+        dfree(dirs);
         dfree(cnt);
         dfree(fill);
         dfree(tsum);
@@ -1071,13 +1075,13 @@ static cudaError_t build_maps(pfem2gpu_handle* h, size_t nc, size_t nvx, size_t 
     int32_t total = 0;
     if (given) {
         total = v2c_offsets[nvx];
-        BM(dalloc(&h->v2c_cells, std::max<size_t>(total, 1)));
-        BM(dalloc(&h->v2c_dirs, std::max<size_t>((size_t)total * dim, 1)));
+        BM(dalloc(&cells, std::max<size_t>(total, 1)));
+        BM(dalloc(&dirs, std::max<size_t>((size_t)total * dim, 1)));
         BM(cudaMemcpyAsync(h->v2c_off, v2c_offsets, (nvx + 1) * 4, cudaMemcpyHostToDevice, s));
-        BM(cudaMemcpyAsync(h->v2c_cells, v2c_cells, (size_t)total * 4, cudaMemcpyHostToDevice, s));
-        BM(cudaMemcpyAsync(h->v2c_dirs, v2c_dirs, (size_t)total * dim * 8, cudaMemcpyHostToDevice, s));
+        BM(cudaMemcpyAsync(cells, v2c_cells, (size_t)total * 4, cudaMemcpyHostToDevice, s));
+        BM(cudaMemcpyAsync(dirs, v2c_dirs, (size_t)total * dim * 8, cudaMemcpyHostToDevice, s));
         BM(dalloc(&h->v2c_rec, std::max<size_t>((size_t)total * 4, 4)));
-        launch_v2c_pack(dim, (size_t)total, h->v2c_cells, h->v2c_dirs, h->v2c_rec, s);
+        launch_v2c_pack(dim, (size_t)total, cells, dirs, h->v2c_rec, s);
         BM(cudaGetLastError());
         BM(cudaStreamSynchronize(s));
         return done(cudaSuccess);
@@ -1089,12 +1093,11 @@ static cudaError_t build_maps(pfem2gpu_handle* h, size_t nc, size_t nvx, size_t 
     BM(cudaGetLastError());
     BM(cudaMemcpyAsync(&total, h->v2c_off + nvx, 4, cudaMemcpyDeviceToHost, s));
     BM(cudaStreamSynchronize(s));
-    BM(dalloc(&h->v2c_cells, std::max<size_t>(total, 1)));
-    BM(dalloc(&h->v2c_dirs, std::max<size_t>((size_t)total * dim, 1)));
-    launch_v2c_build(dim, (int)nc, (int)nvx, h->verts, h->cv, (const uint32_t*)h->v2c_off, fill, h->v2c_cells,
-                     h->v2c_dirs, s);
+    BM(dalloc(&cells, std::max<size_t>(total, 1)));
+    BM(dalloc(&dirs, std::max<size_t>((size_t)total * dim, 1)));
+    launch_v2c_build(dim, (int)nc, (int)nvx, h->verts, h->cv, (const uint32_t*)h->v2c_off, fill, cells, dirs, s);
     BM(dalloc(&h->v2c_rec, std::max<size_t>((size_t)total * 4, 4)));
-    launch_v2c_pack(dim, (size_t)total, h->v2c_cells, h->v2c_dirs, h->v2c_rec, s);
+    launch_v2c_pack(dim, (size_t)total, cells, dirs, h->v2c_rec, s);
     BM(cudaGetLastError());
     BM(cudaStreamSynchronize(s));
 #undef BM
@@ -1128,9 +1131,9 @@ int pfem2gpu_set_mesh(pfem2gpu_handle* h, int64_t n_cells, int64_t n_verts, int6
             if (v2c_cells[k] < 0 || v2c_cells[k] >= n_cells) return fail(h, PFEM2GPU_ERR_ARG, "bad v2c cell");
     }
     // release an older mesh (a failure further down leaves no dangling pointer)
-    for (void** p : {(void**)&h->cv, (void**)&h->cd, (void**)&h->v2c_off, (void**)&h->v2c_cells, (void**)&h->d2c_off,
+    for (void** p : {(void**)&h->cv, (void**)&h->cd, (void**)&h->v2c_off, (void**)&h->d2c_off,
                      (void**)&h->d2c_ent, (void**)&h->verts, (void**)&h->cellX, (void**)&h->aff,
-                     (void**)&h->v2c_dirs, (void**)&h->v2c_rec, (void**)&h->Va, (void**)&h->geo32, (void**)&h->Vstage,
+                     (void**)&h->v2c_rec, (void**)&h->Va, (void**)&h->geo32, (void**)&h->Vstage,
                      (void**)&h->Vstage2,
                      (void**)&h->Vout, (void**)&h->Vin, (void**)&h->Vc, (void**)&h->dVc, (void**)&h->head, (void**)&h->cs0,
                      (void**)&h->cs1, (void**)&h->carr, (void**)&h->carrs, (void**)&h->ccount, (void**)&h->cocc,
@@ -2290,9 +2293,14 @@ int pfem2gpu_get_vertex_maps(pfem2gpu_handle* h, int32_t* offsets, int32_t* cell
     CK(cudaStreamSynchronize(h->stream));
     *n = total;
     if ((cells || dirs) && capacity < total) return fail(h, PFEM2GPU_ERR_ARG, "output arrays too small");
-    if (cells) CK(cudaMemcpyAsync(cells, h->v2c_cells, (size_t)total * 4, cudaMemcpyDeviceToHost, h->stream));
-    if (dirs) CK(cudaMemcpyAsync(dirs, h->v2c_dirs, (size_t)total * h->dim * 8, cudaMemcpyDeviceToHost, h->stream));
+    if (!cells && !dirs) return PFEM2GPU_OK;
+    std::vector<double> rec((size_t)total * 4);  // directions, then the cell in the low half
+    CK(cudaMemcpyAsync(rec.data(), h->v2c_rec, rec.size() * 8, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    for (size_t k = 0; k < (size_t)total; ++k) {
+        if (cells) std::memcpy(cells + k, &rec[4 * k + h->dim], 4);
+        if (dirs) std::memcpy(dirs + k * h->dim, &rec[4 * k], (size_t)h->dim * 8);
+    }
     return PFEM2GPU_OK;
 }
 
