@@ -532,7 +532,7 @@ struct AdvRecStage {
 // V - Vold) and the affine inverses of the chunk's cells.  The loads of these
 // (24 + 24 + 12 doubles a particle, the first 24 in every sub-step) from
 // global memory held every warp for 4 of its 11 cycles per instruction.
-// MAXC cells hold a chunk of 128 particles from 18 to a cell on.
+// MAXC cells hold a chunk of 128 particles from 19 to a cell on.
 struct __align__(16) AdvLin64Stage {
     static constexpr int MAXC = 8, VW = 32, AW = 12;
     double v[MAXC][VW];

@@ -330,7 +330,7 @@ __device__ __forceinline__ bool mild_quad64(const double (*X)[2], const double* 
 // Newton iterations (two thirds of a warp's FP64 operations where one lane
 // in five crosses a face) only told that the point is outside.  Turek mesh,
 // 1.9 M particles, 412 k crossings a step: advect of the FP64 form 201 -> 149
-// us, relocation of the FP32 form 83 -> 76, of the FP64 form 99 -> 93 (85 now).
+// us, relocation of the FP32 form 83 -> 76, of the FP64 form 99 -> 93.
 template <int DIM>
 __device__ __forceinline__ int inverse_map64(const double (*X)[DIM], const double* __restrict__ aff,
                                              const double* p, double* xi_out, bool mild = false)
@@ -456,7 +456,10 @@ __device__ __forceinline__ int inverse_affine64(const double* __restrict__ aff, 
 // passes Newton's first test (|J^-1 f|^2 <= 1e-22), and a guess more than 1e-9
 // outside leads, after clamping, to one Newton step that lands within 1e-11
 // of it and stops.  What is left out is the residual F(g) - p, the Jacobian
-// and its inverse: 250 of the 340 FP64 operations of a sub-step.
+// and its inverse: 250 of the 340 FP64 operations of a sub-step.  LIN64_MAX is
+// about half of that 1e-11 / sqrt(3).  One cell beyond it leaves the whole mesh
+// to Newton: the bound grows with max |x| / h, and of a duct 8 long and 1 wide
+// 128x32x32 cells are within it (2.86e-12) and 136x34x34 are not (3.04e-12).
 constexpr double LIN64_MAX = 3e-12;
 template <typename Aff>  // aff(j): the cell's j-th affine value
 __device__ __forceinline__ int locate_lin64(Aff&& aff, const double* p, double* xi)

@@ -6,9 +6,11 @@
 // arrivals are gathered behind it, and the block then works on these entries
 // one per thread: part counts, survivors of over-full parts (by key), places
 // in the new layout (stayers by a prefix of their survival bits, arrivals by
-// their key), stores.  Nothing is read from global memory twice, and a
-// warp's lanes are all in use whatever a cell holds.  At last a warp per cell
-// takes the partial sums from the staged entries in the new order.
+// their key), stores.  A particle that stays in its cell is read from global
+// memory once, one that changed it twice (with its old cell's slots, and as an
+// arrival), and a warp's lanes are all in use whatever a cell holds.  At last
+// a warp per cell takes the partial sums from the staged entries in the new
+// order.
 //
 // What bounds it, and why tiles.  A time step's memory traffic here is 69
 // bytes a particle (FP32, 3D): 73 us for 7 M at the HBM rate.  One warp per
@@ -16,8 +18,11 @@
 // lanes to cells of 33 or 97 particles, could stage four cells only at
 // seeding density, re-read the written particles for the partial sums of
 // cells above 32, and sent cells above 96 to a path that counts positions
-// through global scratch.  A run settles near 1.9 particles per part (54 a
-// cell at 27 parts, 124 at 64), so those were the paths in use.  Measured,
+// through global scratch.  A run seeded with one particle a part and max 2
+// fills towards 1.9 a part (54 a cell at 27 parts, 124 at 64) at a pace that
+// depends on the flow: after 500 steps a 12^3 cube holds 1.83, a 64x16 channel
+// 1.49 and a 32x8x8 duct 1.20 (1.47 after 1200), so full cells take those
+// paths, and runs stay between the two densities for long (LIGHT).  Measured,
 // before -> now: duct FP32 (7.0 M particles) 480 -> 199 us, FP64 940 -> 406;
 // cube FP32 (32 M) 8414 -> 917, 37^3 cube FP64 (6.2 M) 3253 -> 373; Turek
 // mesh FP32 (1.9 M) 291 -> 91, FP64 429 -> 140.  Now bound by instruction
