@@ -585,15 +585,14 @@ struct ShapeF {
 // left for states read ahead: the backward of a 64x20x20 duct (1.4 M, 10
 // steps) takes 1747 us in FP32 and 2779 in FP64 at 3 blocks and 168 registers
 // without them, 1905 and 2838 with one sub-step's, 2196 and 3134 with 2 blocks
-// and no spill; of a 30^3 cube 4273 us in FP64 (4348 with one ahead), and in
-// FP32 2323 at 4 blocks, 2482 at 3.
-template <int DIM, typename Real, bool AFF>
+// and no spill; of a 30^3 cube 4273 us in FP64 (4348 with one ahead).
+template <int DIM>
 struct WinRev {
-    static constexpr int BLOCKS = DIM == 2 ? 5 : std::is_same<Real, float>::value && !AFF ? 4 : 3;
+    static constexpr int BLOCKS = DIM == 2 ? 5 : 3, MORE = DIM == 2 ? 5 : 4;  // MORE: rev_four
     static constexpr int PF = DIM == 2 ? 2 : 0;  // sub-steps read ahead
 };
-template <int DIM, typename Real, bool AFF>
-__global__ void __launch_bounds__(128, (WinRev<DIM, Real, AFF>::BLOCKS)) k_win_rev(const __grid_constant__ WinArgs w, int j)
+template <int DIM, typename Real, bool AFF, int BLOCKS = WinRev<DIM>::BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) k_win_rev(const __grid_constant__ WinArgs w, int j)
 {
     constexpr int NV = 1 << DIM, NVD = NV * DIM, VS = Dims<DIM>::VS;
     __shared__ double fbuf_s[4][WinFlush<NVD>::ROWS * WF_ROW];
@@ -660,7 +659,7 @@ __global__ void __launch_bounds__(128, (WinRev<DIM, Real, AFF>::BLOCKS)) k_win_r
             }
         }
         // The recorded states stream from HBM and come PF sub-steps ahead, where there is room for them.
-        constexpr int PF = WinRev<DIM, Real, AFF>::PF, LAST = PF > 0 ? PF - 1 : 0;
+        constexpr int PF = WinRev<DIM>::PF, LAST = PF > 0 ? PF - 1 : 0;
         uint32_t pc[LAST + 1];
         Real px[LAST + 1][DIM];
 #pragma unroll
@@ -856,6 +855,22 @@ inline int win_forward_t(const WinArgs& w, cudaStream_t s)
     return n;
 }
 
+// FP32 form, twisted hexes: 4 blocks an SM at 128 registers where that saves a
+// round of blocks against 3 at 168, which spill less.  Reverse sweep of a cube
+// of n^3 cells (2 sub-steps of 4, 2 particles in each of 27 parts), us a segment
+// with 4 and with 3: n = 7 22.9, 23.0; 10 31, 26; 12 50, 46; 14 59, 69; 16 87,
+// 93; 20 162, 177; 30 506, 568.  (12 takes two rounds either way.)
+template <int DIM, typename Real>
+inline bool rev_four(const WinArgs& w)
+{
+    if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
+        const auto rounds = [&](int grid) { return ((long long)w.n + 128ll * grid - 1) / (128ll * grid); };
+        return rounds(win_grid(k_win_rev<DIM, Real, false, WinRev<DIM>::MORE>, 128)) <
+               rounds(win_grid(k_win_rev<DIM, Real, false>, 128));
+    }
+    return false;
+}
+
 // Segments in reverse: replay (recording) unless the record buffer holds the
 // segment already (rec_seg), then the reverse sweep.
 template <int DIM, typename Real>
@@ -868,10 +883,10 @@ inline int win_backward_t(const WinArgs& w, double* g_v0, int rec_seg, cudaStrea
         const int k0 = j * w.C, k1 = k0 + w.C < w.K ? k0 + w.C : w.K;
         if (j != rec_seg)
             for (int k = k0; k < k1; ++k) n += win_step<DIM, Real, true>(w, k, k0, 1, s);
-        if (w.a.mesh.all_affine)
-            k_win_rev<DIM, Real, true><<<win_grid(k_win_rev<DIM, Real, true>, 128), 128, 0, s>>>(w, j);
-        else
-            k_win_rev<DIM, Real, false><<<win_grid(k_win_rev<DIM, Real, false>, 128), 128, 0, s>>>(w, j);
+        const auto reverse = [&](auto* kernel) { kernel<<<win_grid(kernel, 128), 128, 0, s>>>(w, j); };
+        if (w.a.mesh.all_affine) reverse(k_win_rev<DIM, Real, true>);
+        else if (rev_four<DIM, Real>(w)) reverse(k_win_rev<DIM, Real, false, WinRev<DIM>::MORE>);
+        else reverse(k_win_rev<DIM, Real, false>);
         n += 1;
     }
     return n;

@@ -7,6 +7,7 @@ import dataclasses
 import numpy as np
 import pytest
 
+from . import cases
 from .test_gpu_adjoint import CASES, G_RTOL_FP64, objective, rel, setup
 
 pytestmark = pytest.mark.gpu
@@ -47,3 +48,23 @@ def test_fp64_short_segments(which, substeps, K, C, correct):
     assert rel(gV, gV_o) <= G_RTOL_FP64
     if correct:
         assert rel(gVo, gVo_o) <= G_RTOL_FP64
+
+
+@pytest.mark.parametrize("n", [12, 13, 15, 17])
+def test_fp32_twisted_hexes_blocks_per_sm(n):
+    """Sizes on both sides of the choice of 3 or 4 blocks an SM on 148 SMs: 27 n^3 particles are one round of 3,
+    one of 4, two of either, two of 4."""
+    c = cases.cube(n, q=(3, 3, 3), dt=0.3 / n)
+    o, _ = setup(c, "fp64", pre_steps=0)
+    _, g32 = setup(c, "fp32", pre_steps=0)
+    K, C = 3, 2
+    U0 = o.window_forward(K, c.V, c.Vold)
+    gU = objective(U0)[1](U0)
+    _, gv0_o, gV_o, gVo_o = o.window_adjoint(K, c.V, gU, Vold=c.Vold)
+    _, gv0, gV, gVo = g32.adjoint(K, C, c.V, gU, Vold=c.Vold)
+    po, p32 = o.particles(), g32.particles()
+    assert len(p32["id"]) == 27 * n**3
+    oo, og = np.argsort(po["id"]), np.argsort(p32["id"])
+    assert rel(gv0[og], gv0_o[oo]) <= 1e-4
+    assert rel(gV, gV_o) <= 1e-4
+    assert rel(gVo, gVo_o) <= 1e-4
