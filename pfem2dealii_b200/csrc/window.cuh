@@ -180,8 +180,11 @@ __device__ __forceinline__ bool win_relocate(const WinArgs& w, uint32_t& c, Real
 #pragma unroll
         for (int d = 0; d < DIM; ++d) xo.v[d] = (double)xi[d];
         velocity_from_dofs<DIM>(a.mesh.cd, a.Va, c, xo.v, ue.v);
-        const SearchOut so = a.mesh.all_affine ? fallback64<DIM, true>(a.mesh, c, xo, ue, a.pp.dtp)
-                                               : fallback64<DIM, false>(a.mesh, c, xo, ue, a.pp.dtp);
+        // 3D: a copy.  The relocation is a call there and takes the mesh by reference, and reads through a pointer
+        // into the kernel's parameters are slower (FP32 windows on cubes of 9^3 to 19^3 cells: 1 % of the whole pass)
+        const std::conditional_t<DIM == 3, MeshDev, const MeshDev&> mesh = a.mesh;
+        const SearchOut so = mesh.all_affine ? fallback64<DIM, true>(mesh, c, xo, ue, a.pp.dtp)
+                                             : fallback64<DIM, false>(mesh, c, xo, ue, a.pp.dtp);
         if (!(so.flags & SRCH_FOUND)) return false;
         c = so.cell;
 #pragma unroll
