@@ -588,14 +588,19 @@ struct ShapeF {
 // left for states read ahead: the backward of a 64x20x20 duct (1.4 M, 10
 // steps) takes 1747 us in FP32 and 2779 in FP64 at 3 blocks and 168 registers
 // without them, 1905 and 2838 with one sub-step's, 2196 and 3134 with 2 blocks
-// and no spill; of a 30^3 cube 4273 us in FP64 (4348 with one ahead).
+// and no spill; of a 30^3 cube 4273 us in FP64 (4348 with one ahead).  On
+// twisted hexes the vertices are loaded value by value there: a row in 16-byte
+// loads holds 48 registers at once and spills them in every sub-step.  FP32, 30^3
+// cube, us a segment of 4 / 15 / 25 sub-steps: 382 / 905 / 1372 by rows, 358 /
+// 813 / 1214 by values; 4 blocks and 128 registers 341 / 856 / 1294 and 355 /
+// 877 / 1345.  14^3 cube, 15 sub-steps: 110 by rows, 98 by values.
 template <int DIM>
 struct WinRev {
-    static constexpr int BLOCKS = DIM == 2 ? 5 : 3, MORE = DIM == 2 ? 5 : 4;  // MORE: rev_four
+    static constexpr int BLOCKS = DIM == 2 ? 5 : 3;
     static constexpr int PF = DIM == 2 ? 2 : 0;  // sub-steps read ahead
 };
-template <int DIM, typename Real, bool AFF, int BLOCKS = WinRev<DIM>::BLOCKS>
-__global__ void __launch_bounds__(128, BLOCKS) k_win_rev(const __grid_constant__ WinArgs w, int j)
+template <int DIM, typename Real, bool AFF>
+__global__ void __launch_bounds__(128, WinRev<DIM>::BLOCKS) k_win_rev(const __grid_constant__ WinArgs w, int j)
 {
     constexpr int NV = 1 << DIM, NVD = NV * DIM, VS = Dims<DIM>::VS;
     __shared__ double fbuf_s[4][WinFlush<NVD>::ROWS * WF_ROW];
@@ -778,7 +783,14 @@ __global__ void __launch_bounds__(128, BLOCKS) k_win_rev(const __grid_constant__
                 }
             } else {
                 double X[NV][DIM], Ja[DIM][DIM], G[NV][DIM];
-                load_cell64<DIM>(m.cellX, ca, X);
+                if constexpr (DIM == 3) {  // value by value (above)
+#pragma unroll
+                    for (int i = 0; i < NV; ++i)
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) X[i][d] = __ldg(m.cellX + ((size_t)ca * NV + i) * DIM + d);
+                } else {
+                    load_cell64<DIM>(m.cellX, ca, X);
+                }
 #pragma unroll
                 for (int i = 0; i < NV; ++i) sf.value_and_grad(i, G[i]);
 #pragma unroll
@@ -858,22 +870,6 @@ inline int win_forward_t(const WinArgs& w, cudaStream_t s)
     return n;
 }
 
-// FP32 form, twisted hexes: 4 blocks an SM at 128 registers where that saves a
-// round of blocks against 3 at 168, which spill less.  Reverse sweep of a cube
-// of n^3 cells (2 sub-steps of 4, 2 particles in each of 27 parts), us a segment
-// with 4 and with 3: n = 7 22.9, 23.0; 10 31, 26; 12 50, 46; 14 59, 69; 16 87,
-// 93; 20 162, 177; 30 506, 568.  (12 takes two rounds either way.)
-template <int DIM, typename Real>
-inline bool rev_four(const WinArgs& w)
-{
-    if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
-        const auto rounds = [&](int grid) { return ((long long)w.n + 128ll * grid - 1) / (128ll * grid); };
-        return rounds(win_grid(k_win_rev<DIM, Real, false, WinRev<DIM>::MORE>, 128)) <
-               rounds(win_grid(k_win_rev<DIM, Real, false>, 128));
-    }
-    return false;
-}
-
 // Segments in reverse: replay (recording) unless the record buffer holds the
 // segment already (rec_seg), then the reverse sweep.
 template <int DIM, typename Real>
@@ -888,7 +884,6 @@ inline int win_backward_t(const WinArgs& w, double* g_v0, int rec_seg, cudaStrea
             for (int k = k0; k < k1; ++k) n += win_step<DIM, Real, true>(w, k, k0, 1, s);
         const auto reverse = [&](auto* kernel) { kernel<<<win_grid(kernel, 128), 128, 0, s>>>(w, j); };
         if (w.a.mesh.all_affine) reverse(k_win_rev<DIM, Real, true>);
-        else if (rev_four<DIM, Real>(w)) reverse(k_win_rev<DIM, Real, false, WinRev<DIM>::MORE>);
         else reverse(k_win_rev<DIM, Real, false>);
         n += 1;
     }

@@ -51,9 +51,8 @@ def test_fp64_short_segments(which, substeps, K, C, correct):
 
 
 @pytest.mark.parametrize("n", [12, 13, 15, 17])
-def test_fp32_twisted_hexes_blocks_per_sm(n):
-    """Sizes on both sides of the choice of 3 or 4 blocks an SM on 148 SMs: 27 n^3 particles are one round of 3,
-    one of 4, two of either, two of 4."""
+def test_fp32_twisted_hexes_sizes(n):
+    """27 n^3 particles: one round of the reverse sweep's blocks (3 an SM on 148 SMs), a little more, two, and more."""
     c = cases.cube(n, q=(3, 3, 3), dt=0.3 / n)
     o, _ = setup(c, "fp64", pre_steps=0)
     _, g32 = setup(c, "fp32", pre_steps=0)
